@@ -25,36 +25,72 @@ __device__ __forceinline__ void to_real(const cx<double> in[12], cx<R> out[12]) 
     for (int k = 0; k < 12; k++) out[k] = {(R)in[k].re, (R)in[k].im};
 }
 
+// ---- API-layout staging ---------------------------------------------------------
+// A site is contiguous in the API layout (12 complexes of a spinor, 36 of
+// its four links) and spread over planes on the device. The import and
+// export kernels move the API side through shared memory: consecutive
+// threads copy consecutive 16-byte complexes, so both sides are whole
+// 512-byte transactions per warp. A site takes an odd number of 16-byte
+// slots there (13, 37), so that the 8 lanes of a 128-byte phase, one site
+// each, fall on distinct banks. The bound is DRAM. At 24^3x48 in FP64 the
+// export, which stored 16 bytes per 192-byte stride and thread, went from
+// 34.5 us to 25.6 us per parity (5.0 TB/s), the import stayed at
+// 22.7 us, the links went from 129 to 119 us (6.4 TB/s); both parities and
+// the links together from 268 to 214 us.
+constexpr int kSpinorSites = 128;  // sites (and threads) of a block
+constexpr int kLinkSites = 32;     // sites of a block of 128 threads, one link each
+
+// complexes of the n sites at `src` -> slots of `per + 1` at `st` (commit and wait included)
+template <int PER, int SITES>
+__device__ __forceinline__ void stage_sites(double2 *st, const double2 *__restrict__ src, int n) {
+    const uint32_t s0 = smem_addr(st);
+#pragma unroll
+    for (int i = threadIdx.x; i < PER * SITES; i += 128)
+        if (i < PER * n) cp_async16_cg(s0 + (uint32_t)(i + i / PER) * 16u, src + i);
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();
+}
+
 // ---- spinors ------------------------------------------------------------------
 template <int PREC>
-__global__ void k_spinor_import(const double2 *__restrict__ aos, long Vh, int parity, void *dst, long first,
-                                long count) {
-    long h = first + (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (h >= first + count) return;
-    const double2 *p = aos + (parity * Vh + h) * 12;
+__global__ void __launch_bounds__(kSpinorSites) k_spinor_import(const double2 *__restrict__ aos, long Vh, int parity,
+                                                                void *dst, long first, long count) {
+    __shared__ double2 st[kSpinorSites * 13];
+    const long b0 = (long)blockIdx.x * kSpinorSites;  // first site of the block, from `first`
+    const int n = (int)min((long)kSpinorSites, count - b0);
+    stage_sites<12, kSpinorSites>(st, aos + (parity * Vh + first + b0) * 12, n);
+    if ((int)threadIdx.x >= n) return;
     cx<double> s[12];
 #pragma unroll
     for (int k = 0; k < 12; k++) {
-        double2 v = p[k];
+        double2 v = st[threadIdx.x * 13 + k];
         s[k] = {v.x, v.y};
     }
     using R = typename SpinorIO<PREC>::real;
     cx<R> r[12];
     to_real(s, r);
-    SpinorIO<PREC>::store(dst, Vh, h, r);
+    SpinorIO<PREC>::store(dst, Vh, first + b0 + threadIdx.x, r);
 }
 
 template <int PREC>
-__global__ void k_spinor_export(const void *src, long Vh, int parity, double2 *__restrict__ aos, long first,
-                                long count) {
-    long h = first + (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (h >= first + count) return;
-    using R = typename SpinorIO<PREC>::real;
-    cx<R> r[12];
-    SpinorIO<PREC>::load(src, Vh, h, r);
-    double2 *p = aos + (parity * Vh + h) * 12;
+__global__ void __launch_bounds__(kSpinorSites) k_spinor_export(const void *src, long Vh, int parity,
+                                                                double2 *__restrict__ aos, long first, long count) {
+    __shared__ double2 st[kSpinorSites * 13];
+    const long b0 = (long)blockIdx.x * kSpinorSites;
+    const int n = (int)min((long)kSpinorSites, count - b0);
+    if ((int)threadIdx.x < n) {
+        using R = typename SpinorIO<PREC>::real;
+        cx<R> r[12];
+        SpinorIO<PREC>::load(src, Vh, first + b0 + threadIdx.x, r);
 #pragma unroll
-    for (int k = 0; k < 12; k++) p[k] = make_double2((double)r[k].re, (double)r[k].im);
+        for (int k = 0; k < 12; k++) st[threadIdx.x * 13 + k] = make_double2((double)r[k].re, (double)r[k].im);
+    }
+    __syncthreads();
+    double2 *p = aos + (parity * Vh + first + b0) * 12;
+#pragma unroll
+    for (int i = threadIdx.x; i < 12 * kSpinorSites; i += kSpinorSites)
+        if (i < 12 * n) st_cs(p + i, st[i + i / 12]);
 }
 
 // split real / imaginary planes: component k of staged site h at re[12*h+k]
@@ -116,23 +152,27 @@ __global__ void k_spinor_gaussian(void *dst, long Vh, int parity, uint64_t seed)
 }
 
 // ---- gauge --------------------------------------------------------------------
+// the four links of the sites [first, first + n) (even/odd index over both
+// parities); `aos` points at the first one. Warp mu of a block stores the
+// direction-mu links of 32 consecutive sites (a block may span the parities)
 template <int PREC, int RECON>
-__global__ void k_gauge_import(const double2 *__restrict__ aos, long first, long n, long Vh, void *dst) {
-    long k = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    long l = first + k;  // global link index 4*i + mu
-    long i = l >> 2;
-    int mu = (int)(l & 3);
-    int par = i >= Vh;
-    long h = i - par * Vh;
-    const double2 *p = aos + k * 9;
+__global__ void __launch_bounds__(4 * kLinkSites) k_gauge_import(const double2 *__restrict__ aos, long first, long n,
+                                                                 long Vh, void *dst) {
+    __shared__ double2 st[kLinkSites * 37];
+    const long b0 = (long)blockIdx.x * kLinkSites;
+    const int nb = (int)min((long)kLinkSites, n - b0);
+    stage_sites<36, kLinkSites>(st, aos + b0 * 36, nb);
+    const int mu = threadIdx.x / kLinkSites, j = threadIdx.x % kLinkSites;
+    if (j >= nb) return;
+    const long i = first + b0 + j;
+    const int par = i >= Vh;
     cx<double> U[9];
 #pragma unroll
     for (int e = 0; e < 9; e++) {
-        double2 v = p[e];
+        double2 v = st[j * 37 + mu * 9 + e];
         U[e] = {v.x, v.y};
     }
-    LinkIO<PREC, RECON>::store(dst, Vh, par, mu, h, U);
+    LinkIO<PREC, RECON>::store(dst, Vh, par, mu, i - par * Vh, U);
 }
 
 // links from split planes: element e of staged link k at re[9*k+e]
@@ -265,7 +305,9 @@ int launch_spinor_import(const Geom &g, cudaStream_t s, const void *aos, int par
     PLQCD_TRY(check_field_ptr(aos, "spinor import (API layout)"));
     PLQCD_TRY(check_field_ptr(dst, "spinor import"));
     if (count < 0) count = g.Vh - first;
-#define F(P) dev::k_spinor_import<P><<<dev::nblocks(count), dev::kBlock, 0, s>>>((const double2 *)aos, g.Vh, parity, dst, first, count)
+    if (count < 1) return set_error(PLQCD_ERR_ARG, "spinor import: %ld sites", count);
+    const unsigned nb = (unsigned)((count + dev::kSpinorSites - 1) / dev::kSpinorSites);
+#define F(P) dev::k_spinor_import<P><<<nb, dev::kSpinorSites, 0, s>>>((const double2 *)aos, g.Vh, parity, dst, first, count)
     PLQCD_SPINOR_SWITCH(prec, F)
 #undef F
     PLQCD_CUDA_TRY(cudaGetLastError());
@@ -277,7 +319,9 @@ int launch_spinor_export(const Geom &g, cudaStream_t s, const void *src, int pre
     PLQCD_TRY(check_field_ptr(src, "spinor export"));
     PLQCD_TRY(check_field_ptr(aos, "spinor export (API layout)"));
     if (count < 0) count = g.Vh - first;
-#define F(P) dev::k_spinor_export<P><<<dev::nblocks(count), dev::kBlock, 0, s>>>(src, g.Vh, parity, (double2 *)aos, first, count)
+    if (count < 1) return set_error(PLQCD_ERR_ARG, "spinor export: %ld sites", count);
+    const unsigned nb = (unsigned)((count + dev::kSpinorSites - 1) / dev::kSpinorSites);
+#define F(P) dev::k_spinor_export<P><<<nb, dev::kSpinorSites, 0, s>>>(src, g.Vh, parity, (double2 *)aos, first, count)
     PLQCD_SPINOR_SWITCH(prec, F)
 #undef F
     PLQCD_CUDA_TRY(cudaGetLastError());
@@ -341,7 +385,10 @@ int launch_spinor_gaussian(const Geom &g, cudaStream_t s, void *dst, int prec, i
 int launch_gauge_import(const Geom &g, cudaStream_t s, const void *aos, long first, long n, void *dst, int prec,
                         int recon) {
     PLQCD_TRY(check_field_ptr(aos, "gauge import (API layout)"));
-#define F(P, R) dev::k_gauge_import<P, R><<<dev::nblocks(n), dev::kBlock, 0, s>>>((const double2 *)aos, first, n, g.Vh, dst)
+    if (first < 0 || n < 4 || first % 4 || n % 4 || first + n > 8 * g.Vh)
+        return set_error(PLQCD_ERR_ARG, "gauge import: links [%ld, %ld) are not whole sites", first, first + n);
+    const unsigned nb = (unsigned)((n / 4 + dev::kLinkSites - 1) / dev::kLinkSites);
+#define F(P, R) dev::k_gauge_import<P, R><<<nb, 4 * dev::kLinkSites, 0, s>>>((const double2 *)aos, first / 4, n / 4, g.Vh, dst)
     PLQCD_GAUGE_SWITCH(prec, recon, F)
 #undef F
     PLQCD_CUDA_TRY(cudaGetLastError());
