@@ -30,88 +30,56 @@
 #include "tune.h"
 
 namespace plqcd {
+
+int launch_dslash_ahead(cudaStream_t s, const dev::DslashArgs &a, int prec, int recon, bool xpay, bool full,
+                        int variant);
+
 namespace dev {
 
-// One direction (MU, FWD) of one output site.
-template <class SIO, class LIO, int MU, bool FWD, bool COMPAT>
-__device__ __forceinline__ void hop_dir(cx<typename SIO::real> acc[12], const void *in, const void *gauge,
-                                        long Vh, long h_nbr, int link_par, long h_link,
-                                        typename SIO::real sg_in) {
+// Direct loads at the use, for the reference's as-shipped results (COMPAT,
+// FP64, one parity): a check, not a path whose speed matters. Everything
+// else loads ahead (dslash_ahead.cu).
+template <class SIO, class LIO>
+__global__ void __launch_bounds__(256) k_dslash_compat(const DslashArgs a) {
     using R = typename SIO::real;
-    cx<R> s[12];
-    R n;
-    SIO::load_raw(in, Vh, h_nbr, s, n);
-    cx<R> U[9];
-    LIO::load(gauge, Vh, link_par, MU, h_link, U);
-    // projection, SU(3) product and rebuild (with COMPAT, the reference's
-    // as-shipped loss of the forward terms of spins 2, 3)
-    compute_dir_n<COMPAT, SIO::kScaled, R>(FWD ? MU : MU + 4, acc, s, U, sg_in, n);
-}
-
-template <class SIO, class LIO, bool COMPAT, bool XPAY, bool FULL>
-__global__ void __launch_bounds__(256) k_dslash(const DslashArgs a) {
-    using R = typename SIO::real;
-    int par;
-    long h;
-    if (FULL) {
-        par = blockIdx.x & 1;
-        h = (long)(blockIdx.x >> 1) * blockDim.x + threadIdx.x;
-    } else {
-        par = a.out_parity;
-        h = a.h_begin + (long)(blockIdx.x / a.nrhs) * blockDim.x + threadIdx.x;
-    }
+    const int par = a.out_parity;
+    const long h = a.h_begin + (long)(blockIdx.x / a.nrhs) * blockDim.x + threadIdx.x;
     if (h >= a.h_end) return;
-    // selects, not a dynamic index into the parameter arrays (which would
-    // copy them to local memory)
-    const long roff = FULL ? 0 : (long)(blockIdx.x % a.nrhs) * a.fbytes;  // RHS of this block
-    const void *in = (FULL && par == 0) ? a.in[1] : static_cast<const char *>(a.in[0]) + roff;
-    void *out = (FULL && par == 1) ? a.out[1] : static_cast<char *>(a.out[0]) + roff;
+    const long roff = (long)(blockIdx.x % a.nrhs) * a.fbytes;  // RHS of this block
+    const void *in = static_cast<const char *>(a.in[0]) + roff;
+    void *out = static_cast<char *>(a.out[0]) + roff;
     const long Vh = a.Vh;
-    const int L0h = a.L0h, L1 = a.L1, L2 = a.L2, L3 = a.L3;
-    const Coords c = site_coords(h, par, L0h, L1, L2);
-    const int xh = (int)(h - c.row * L0h);
-
-    // neighbour half-site indices (periodic wrap on the device)
-    int nbs[8];
-    neighbour_sites(c, xh, a.L0, L0h, L1, L2, L3, nbs);
-    const int h_xp = nbs[0], h_yp = nbs[1], h_zp = nbs[2], h_tp = nbs[3];
-    const int h_xm = nbs[4], h_ym = nbs[5], h_zm = nbs[6], h_tm = nbs[7];
+    const Coords c = site_coords(h, par, a.L0h, a.L1, a.L2);
+    const int xh = (int)(h - c.row * a.L0h);
+    int nb[8];
+    neighbour_sites(c, xh, a.L0, a.L0h, a.L1, a.L2, a.L3, nb);
 
     const R sg = (R)a.g5_in;
     const int opp = par ^ 1;
     // as shipped, oe takes forward links of odd site h from the even site
     // with the same half index (lib/dirac.c:643)
-    const int fpar = (COMPAT && par == 1) ? 0 : par;
+    const int fpar = 0;
 
     cx<R> acc[12];
 #pragma unroll
     for (int k = 0; k < 12; k++) acc[k] = {R(0), R(0)};
-
-    // the order of dir_at: x+, x-, y+, y-, z+, z-, t+, t-
-    hop_dir<SIO, LIO, 0, true, COMPAT>(acc, in, a.gauge, Vh, h_xp, fpar, h, sg);
-    hop_dir<SIO, LIO, 0, false, COMPAT>(acc, in, a.gauge, Vh, h_xm, opp, h_xm, sg);
-    hop_dir<SIO, LIO, 1, true, COMPAT>(acc, in, a.gauge, Vh, h_yp, fpar, h, sg);
-    hop_dir<SIO, LIO, 1, false, COMPAT>(acc, in, a.gauge, Vh, h_ym, opp, h_ym, sg);
-    hop_dir<SIO, LIO, 2, true, COMPAT>(acc, in, a.gauge, Vh, h_zp, fpar, h, sg);
-    hop_dir<SIO, LIO, 2, false, COMPAT>(acc, in, a.gauge, Vh, h_zm, opp, h_zm, sg);
-    hop_dir<SIO, LIO, 3, true, COMPAT>(acc, in, a.gauge, Vh, h_tp, fpar, h, sg);
-    hop_dir<SIO, LIO, 3, false, COMPAT>(acc, in, a.gauge, Vh, h_tm, opp, h_tm, sg);
-
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        const int d = dir_at(k);
+        cx<R> s[12], U[9];
+        R n;
+        SIO::load_raw(in, Vh, nb[d], s, n);
+        if (d < 4)
+            LIO::load(a.gauge, Vh, fpar, d, h, U);
+        else
+            LIO::load(a.gauge, Vh, opp, d - 4, nb[d], U);
+        compute_dir_n<true, SIO::kScaled, R>(d, acc, s, U, sg, n);
+    }
     const R aup = (R)a.a_up, alow = (R)a.a_low;
-    if (XPAY) {
-        cx<R> xv[12];
-        SIO::load(static_cast<const char *>(a.x) + roff, Vh, h, xv);
-        const R b = (R)a.b;
 #pragma unroll
-        for (int k = 0; k < 12; k++) {
-            const R ak = k < 6 ? aup : alow;
-            acc[k] = {fma(ak, acc[k].re, b * xv[k].re), fma(ak, acc[k].im, b * xv[k].im)};
-        }
-    } else {
-#pragma unroll
-        for (int k = 6; k < 12; k++) acc[k] = {alow * acc[k].re, alow * acc[k].im};
-#pragma unroll
-        for (int k = 0; k < 6; k++) acc[k] = {aup * acc[k].re, aup * acc[k].im};
+    for (int k = 0; k < 12; k++) {
+        const R ak = k < 6 ? aup : alow;
+        acc[k] = {ak * acc[k].re, ak * acc[k].im};
     }
     SIO::store(out, Vh, h, acc);
 }
@@ -218,151 +186,21 @@ static int launch_pipe(const Geom &g, cudaStream_t s, const DslashArgs &a, int b
     return PLQCD_OK;
 }
 
-// Two sites per thread (sites h and h + blockDim of a 2*blockDim tile),
-// direct loads, the direction loops of both sites interleaved: twice the
-// independent loads in flight per thread and shared index arithmetic, for
-// the 32- and 16-bit formats whose kernels are latency / issue bound.
-// PACK: the two sites are the two lanes of packed FP32 instructions (f2),
-// which halves the arithmetic instructions and gives the same bits.
-// Single parity only (RHS blocks allowed), no bug-compatible mode.
-template <class SIO, class LIO, bool XPAY, bool PACK>
-__global__ void __launch_bounds__(256) k_dslash_spt2(const DslashArgs a) {
-    using R = typename SIO::real;
-    constexpr int S = 2;
-    const int par = a.out_parity, opp = par ^ 1;
-    const long tile = blockIdx.x / a.nrhs;
-    const long roff = (long)(blockIdx.x % a.nrhs) * a.fbytes;
-    const void *in = static_cast<const char *>(a.in[0]) + roff;
-    void *out = static_cast<char *>(a.out[0]) + roff;
-    const long Vh = a.Vh;
-    const int L0h = a.L0h, L1 = a.L1, L2 = a.L2, L3 = a.L3;
-    long hs[S];
-    int nb[S][8];
-    bool ok[S];
-#pragma unroll
-    for (int j = 0; j < S; j++) {
-        long h = a.h_begin + tile * (S * blockDim.x) + j * blockDim.x + threadIdx.x;
-        ok[j] = h < a.h_end;
-        if (!ok[j]) h = a.h_begin;  // compute on a valid site, store nothing
-        hs[j] = h;
-        const Coords c = site_coords(h, par, L0h, L1, L2);
-        const int xh = (int)(h - c.row * L0h);
-        neighbour_sites(c, xh, a.L0, L0h, L1, L2, L3, nb[j]);
-    }
-    if (!ok[0]) return;
-    const R sg = (R)a.g5_in;
-    cx<R> acc[S][12];
-    if constexpr (PACK) {
-        static_assert(S == 2, "one site per lane");
-        cx<f2> acc2[12];
-#pragma unroll
-        for (int k = 0; k < 12; k++) acc2[k] = {f2(0.f), f2(0.f)};
-        const f2 sg2(sg);
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-            const int d = dir_at(k);
-            cx<R> s[S][12], U[S][9];
-            R n[S];
-#pragma unroll
-            for (int j = 0; j < S; j++) {
-                SIO::load_raw(in, Vh, nb[j][d], s[j], n[j]);
-                if (d < 4)
-                    LIO::load(a.gauge, Vh, par, d, hs[j], U[j]);
-                else
-                    LIO::load(a.gauge, Vh, opp, d - 4, nb[j][d], U[j]);
-            }
-            cx<f2> s2[12], U2[9];
-#pragma unroll
-            for (int k = 0; k < 12; k++) s2[k] = zip(s[0][k], s[1][k]);
-#pragma unroll
-            for (int k = 0; k < 9; k++) U2[k] = zip(U[0][k], U[1][k]);
-            compute_dir_n<false, SIO::kScaled, f2>(d, acc2, s2, U2, sg2, f2(n[0], n[1]));
-        }
-#pragma unroll
-        for (int j = 0; j < S; j++)
-#pragma unroll
-            for (int k = 0; k < 12; k++) acc[j][k] = lane(acc2[k], j);
-    } else {
-#pragma unroll
-        for (int j = 0; j < S; j++)
-#pragma unroll
-            for (int k = 0; k < 12; k++) acc[j][k] = {R(0), R(0)};
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-            const int d = dir_at(k);
-            cx<R> s[S][12], U[S][9];
-            R n[S];
-#pragma unroll
-            for (int j = 0; j < S; j++) {
-                SIO::load_raw(in, Vh, nb[j][d], s[j], n[j]);
-                if (d < 4)
-                    LIO::load(a.gauge, Vh, par, d, hs[j], U[j]);
-                else
-                    LIO::load(a.gauge, Vh, opp, d - 4, nb[j][d], U[j]);
-            }
-#pragma unroll
-            for (int j = 0; j < S; j++) compute_dir_n<false, SIO::kScaled, R>(d, acc[j], s[j], U[j], sg, n[j]);
-        }
-    }
-    const R aup = (R)a.a_up, alow = (R)a.a_low;
-#pragma unroll
-    for (int j = 0; j < S; j++) {
-        if (!ok[j]) continue;
-        if (XPAY) {
-            cx<R> xv[12];
-            SIO::load(static_cast<const char *>(a.x) + roff, Vh, hs[j], xv);
-            const R b = (R)a.b;
-#pragma unroll
-            for (int k = 0; k < 12; k++) {
-                const R ak = k < 6 ? aup : alow;
-                acc[j][k] = {fma(ak, acc[j][k].re, b * xv[k].re), fma(ak, acc[j][k].im, b * xv[k].im)};
-            }
-        } else {
-#pragma unroll
-            for (int k = 0; k < 12; k++) {
-                const R ak = k < 6 ? aup : alow;
-                acc[j][k] = {ak * acc[j][k].re, ak * acc[j][k].im};
-            }
-        }
-        SIO::store(out, Vh, hs[j], acc[j]);
-    }
-}
-
+// variant 2, 3: cp.async pipeline of that depth; anything else: loads ahead
+// in registers (20, 21, 22 of dslash_ahead.cu; tuning files may still hold
+// 0, 12 and 13, kernels that it replaced)
 template <class SIO, class LIO, bool COMPAT, bool XPAY, bool FULL>
-static int launch_direct(const Geom &g, cudaStream_t s, const DslashArgs &a, int block);
-
-template <class SIO, class LIO, bool COMPAT, bool XPAY, bool FULL>
-static int launch_spt2(const Geom &g, cudaStream_t s, const DslashArgs &a, int block, bool pack) {
-    if constexpr (COMPAT || FULL || std::is_same<typename SIO::real, double>::value) {
-        return set_error(PLQCD_ERR_ARG, "dslash: two sites per thread exists for 32/16-bit single-parity calls");
-    } else {
-        const long nblk = (a.h_end - a.h_begin + 2L * block - 1) / (2L * block) * a.nrhs;
-        if (pack)
-            k_dslash_spt2<SIO, LIO, XPAY, true><<<(unsigned)nblk, block, 0, s>>>(a);
-        else
-            k_dslash_spt2<SIO, LIO, XPAY, false><<<(unsigned)nblk, block, 0, s>>>(a);
-        PLQCD_CUDA_TRY(cudaGetLastError());
-        return PLQCD_OK;
-    }
-}
-
-// variant 0: direct loads; 2, 3: cp.async pipeline of that depth; 12: two
-// sites per thread; 13: the same on packed FP32 lanes
-template <class SIO, class LIO, bool COMPAT, bool XPAY, bool FULL>
-static int launch_t(const Geom &g, cudaStream_t s, const DslashArgs &a, int variant, int block) {
+static int launch_t(const Geom &g, cudaStream_t s, const DslashArgs &a, int prec, int recon, int variant, int block) {
     if (variant == 2) return launch_pipe<SIO, LIO, 2, COMPAT, XPAY, FULL>(g, s, a, block);
     if (variant == 3) return launch_pipe<SIO, LIO, 3, COMPAT, XPAY, FULL>(g, s, a, block);
-    if (variant == 12 || variant == 13) return launch_spt2<SIO, LIO, COMPAT, XPAY, FULL>(g, s, a, block, variant == 13);
-    return launch_direct<SIO, LIO, COMPAT, XPAY, FULL>(g, s, a, block);
-}
-
-template <class SIO, class LIO, bool COMPAT, bool XPAY, bool FULL>
-static int launch_direct(const Geom &g, cudaStream_t s, const DslashArgs &a, int block) {
-    long nblk = (a.h_end - a.h_begin + block - 1) / block * a.nrhs;
-    if (FULL) nblk *= 2;
-    k_dslash<SIO, LIO, COMPAT, XPAY, FULL><<<(unsigned)nblk, block, 0, s>>>(a);
-    PLQCD_CUDA_TRY(cudaGetLastError());
-    return PLQCD_OK;
+    if constexpr (COMPAT) {
+        const long nblk = (a.h_end - a.h_begin + block - 1) / block * a.nrhs;
+        k_dslash_compat<SIO, LIO><<<(unsigned)nblk, block, 0, s>>>(a);
+        PLQCD_CUDA_TRY(cudaGetLastError());
+        return PLQCD_OK;
+    } else {
+        return launch_dslash_ahead(s, a, prec, recon, XPAY, FULL, variant);
+    }
 }
 
 template <int PREC, int RECON>
@@ -370,13 +208,13 @@ static int launch_pr(const Geom &g, cudaStream_t s, const DslashArgs &a, int var
                      bool xpay, bool full) {
     using S = SpinorIO<PREC>;
     using L = LinkIO<PREC, RECON>;
-    if (full) return launch_t<S, L, false, false, true>(g, s, a, variant, block);
+    if (full) return launch_t<S, L, false, false, true>(g, s, a, PREC, RECON, variant, block);
     if (compat) {
-        if (PREC == PLQCD_F64 && RECON == 18) return launch_t<S, L, true, false, false>(g, s, a, variant, block);
+        if (PREC == PLQCD_F64 && RECON == 18) return launch_t<S, L, true, false, false>(g, s, a, PREC, RECON, variant, block);
         return set_error(PLQCD_ERR_ARG, "dslash: the bug-compatible mode exists for F64 18-real links only");
     }
-    if (xpay) return launch_t<S, L, false, true, false>(g, s, a, variant, block);
-    return launch_t<S, L, false, false, false>(g, s, a, variant, block);
+    if (xpay) return launch_t<S, L, false, true, false>(g, s, a, PREC, RECON, variant, block);
+    return launch_t<S, L, false, false, false>(g, s, a, PREC, RECON, variant, block);
 }
 
 }  // namespace dev
@@ -424,7 +262,7 @@ int launch_dslash(const Geom &g, cudaStream_t s, const DslashCall &c) {
     // a partial site range (the drop-in path's t-slab chunks) is a separate
     // entry: the TMA kernel takes whole fields only
     const bool part = a.h_begin != 0 || a.h_end != g.Vh;
-    snprintf(key, sizeof key, "%sdslash|p%d|r%d|%s%s%s%s|%dx%dx%dx%d|n%d", device_tag().c_str(), c.prec, c.recon,
+    snprintf(key, sizeof key, "%sdslash|p%d|r%d|%s%s%s%s|%dx%dx%dx%d|n%d|c2", device_tag().c_str(), c.prec, c.recon,
              c.full ? "full" : "half", c.x ? "+xpay" : "", compat ? "+compat" : "", part ? "+range" : "", g.L[0],
              g.L[1], g.L[2], g.L[3], c.nrhs);
     return tune_dslash(g, s, c, a, key);
@@ -475,23 +313,34 @@ static int build_args(const Geom &g, const DslashCall &c, dev::DslashArgs &a) {
 
 static int tune_dslash(const Geom &g, cudaStream_t s, const DslashCall &c, const dev::DslashArgs &a,
                        const char *key) {
-    // load strategy (0 direct, 2/3 cp.async pipeline depth, 12 two sites per
-    // thread) x block size
+    // loads ahead in registers (20, 21, 22), cp.async pipeline depth (2, 3)
+    // x block size. The first one runs where tuning is not possible.
     std::vector<TuneResult> cands;
-    const bool spt_ok = c.prec != PLQCD_F64 && !c.full && !(c.flags & PLQCD_DSLASH_COMPAT);
-    for (int v : {2, 0, 3, 12, 13}) {
-        if (v >= 12 && !spt_ok) continue;
-        for (int b : {64, 128, 256}) {
-            TuneResult r;
-            r.variant = v;
-            r.block = b;
-            cands.push_back(r);
-        }
+    const bool compat = (c.flags & PLQCD_DSLASH_COMPAT) != 0;
+    auto add = [&](int variant, int block) {
+        TuneResult r;
+        r.variant = variant;
+        r.block = block;
+        cands.push_back(r);
+    };
+    if (compat) {
+        add(2, 64);
+        add(0, 64);
+    } else {
+        if (c.full && c.prec == PLQCD_F64) add(21, 64);
+        if (c.prec != PLQCD_F64) add(22, 64);
+        add(20, 64);
+        for (int v : {2, 3})
+            for (int b : {64, 128, 256}) add(v, b);
     }
     // TMA-staged rows: ring depth x rows per tile, where the tile fits
     const long slab = (long)g.L0h * g.L[1] * g.L[2];  // TMA tiles cover whole t-slices
-    const bool tma_ok = !(c.flags & PLQCD_DSLASH_COMPAT) && c.nrhs == 1 && a.h_begin % slab == 0 &&
-                        (a.h_end - a.h_begin) % slab == 0 && getenv("PLQCD_NO_TMA") == nullptr;
+    // (FP64 full lattice only: with loads ahead in registers the others lose
+    // at every measured size, e.g. F64 xpay at 32^3x64 295 us against 270,
+    // F32-18 full lattice 296 against 180; a near-tie is left at 16^3x32, 32.5
+    // against 32.8)
+    const bool tma_ok = c.full && c.prec == PLQCD_F64 && a.h_begin % slab == 0 && (a.h_end - a.h_begin) % slab == 0 &&
+                        getenv("PLQCD_NO_TMA") == nullptr;
     if (tma_ok)
         // (kinds 3 and 5, two own-line buffers, lost to 2 and 4 at every
         // measured point and are not tried). The own-line kernels (4, 2)
@@ -508,10 +357,7 @@ static int tune_dslash(const Geom &g, cudaStream_t s, const DslashCall &c, const
                         clear_error();
                         continue;
                     }
-                    TuneResult r;
-                    r.variant = 1000 * kind + 100 * ns + ny;
-                    r.block = blk;
-                    cands.push_back(r);
+                    add(1000 * kind + 100 * ns + ny, blk);
                 }
     // trial launches write into scratch outputs: an xpay whose output aliases
     // its x operand must not be applied more than once

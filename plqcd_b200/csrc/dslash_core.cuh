@@ -309,7 +309,8 @@ __device__ __forceinline__ void compute_dir_pk(cx<float> acc[12], const cx<float
 
 // PK: FP32 on packed lanes within the site (compute_dir_pk). It pays in
 // the single-RHS cp.async pipeline kernel (32^3x64: F16 xpay hop -12%, BF16
-// -9%, F32 -1..-4% as tuned) and loses in the direct-load, multi-RHS and TMA
+// -9%, F32 -1..-4% as tuned) and in the kernel that loads ahead into
+// registers (F16 xpay 84 against 88 us), and loses in the multi-RHS and TMA
 // kernels, which keep the scalar form; both give the same bits.
 template <bool COMPAT, bool SC, typename R, bool PK = false>
 __device__ __forceinline__ void compute_dir_n(int d, cx<R> acc[12], const cx<R> s[12], const cx<R> U[9], R sg,

@@ -10,6 +10,9 @@
 //   {"key": "...", "variant": V, "block": B, "ms": T}
 // Tuning is skipped (the first candidate is used) while the stream is being
 // captured into a CUDA graph, or when PLQCD_TUNE=0.
+// A key ends in the number of its candidate list ("|c2"), so an entry of an
+// older file does not hide the kernels that came since; where tuning is
+// skipped, the entry an older file holds for the launch serves after all.
 #include <cuda_runtime.h>
 #include <sys/stat.h>
 
@@ -74,6 +77,17 @@ void save_locked(const std::string &path) {
     rename(tmp.c_str(), path.c_str());
 }
 
+// the entry of `key`, or with `older` of the same launch in a file written
+// before its candidate list was numbered
+bool find_locked(const std::string &key, bool older, TuneResult *out) {
+    auto it = cache().find(key);
+    const size_t c = key.rfind("|c");
+    if (it == cache().end() && older && c != std::string::npos) it = cache().find(key.substr(0, c));
+    if (it == cache().end()) return false;
+    if (out) *out = it->second;
+    return true;
+}
+
 void ensure_loaded_locked() {
     if (!g_loaded) {
         load_locked(default_path());
@@ -113,19 +127,15 @@ int tune_launch(const std::string &key, cudaStream_t s, const std::vector<TuneRe
                 const std::function<int(const TuneResult &, bool)> &run) {
     if (cands.empty()) return set_error(PLQCD_ERR_ARG, "tune: no candidates for %s", key.c_str());
     TuneResult chosen = cands[0];
-    bool found = false;
-    {
-        std::lock_guard<std::mutex> lk(g_mu);
-        ensure_loaded_locked();
-        auto it = cache().find(key);
-        if (it != cache().end()) {
-            chosen = it->second;
-            found = true;
-        }
-    }
-    if (found || !tune_enabled()) return run(chosen, false);
+    if (tune_lookup(key, &chosen) || !tune_enabled()) return run(chosen, false);
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return run(chosen, false);
+    if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+        {
+            std::lock_guard<std::mutex> lk(g_mu);
+            find_locked(key, true, &chosen);
+        }
+        return run(chosen, false);
+    }
 
     cudaEvent_t e0, e1;
     if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess) {
@@ -244,10 +254,7 @@ int tune_launch(const std::string &key, cudaStream_t s, const std::vector<TuneRe
 bool tune_lookup(const std::string &key, TuneResult *out) {
     std::lock_guard<std::mutex> lk(g_mu);
     ensure_loaded_locked();
-    auto it = cache().find(key);
-    if (it == cache().end()) return false;
-    if (out) *out = it->second;
-    return true;
+    return find_locked(key, !tune_enabled(), out);
 }
 
 }  // namespace plqcd

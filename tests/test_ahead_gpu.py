@@ -1,0 +1,75 @@
+"""The kernels that load the next directions into registers: the same bits as
+the cp.async pipeline kernel (whose results the oracle tests check) in every
+format and mode, at half volumes below a block, ragged in the last block, with
+odd half extents, and over site ranges; FP64 also against the oracle."""
+import numpy as np
+import pytest
+
+import plqcd_b200 as P
+from oracle import oracle as O
+from tests.gpu_util import dev_bytes, field_from_host, field_to_host, new_lattice, relmax, to_dev
+
+pytestmark = pytest.mark.gpu
+
+FORMATS = [(P.F64, 18), (P.F64, 12), (P.F32, 18), (P.F32, 12), (P.F16, 12), (P.BF16, 12)]
+# half volumes 8 (a quarter of a warp), 120, 420 and 1440 (blocks of 64 and of 32 sites ragged or not)
+DIMS = [(2, 2, 2, 2), (10, 6, 2, 2), (6, 10, 14, 2), (12, 4, 6, 10)]
+
+
+def _force(monkeypatch, variant):
+    monkeypatch.setenv("PLQCD_DSLASH_STAGES", str(variant))
+    monkeypatch.setenv("PLQCD_DSLASH_BLOCK", "64")
+
+
+@pytest.mark.parametrize("dims", DIMS)
+@pytest.mark.parametrize("prec,recon", FORMATS)
+def test_ahead_same_bits(cuda, monkeypatch, dims, prec, recon):
+    lat = new_lattice(dims)
+    g = P.Gauge(lat, prec, recon)
+    g.random(11)
+    nb = lat.spinor_bytes(prec)
+    n = 3  # right-hand sides of the folded launch
+    fe, fo, x = dev_bytes(n * nb), dev_bytes(n * nb), dev_bytes(n * nb)
+    for r in range(n):
+        lat.spinor_gaussian(fe[r * nb:], prec, 0, 20 + r)
+        lat.spinor_gaussian(fo[r * nb:], prec, 1, 30 + r)
+        lat.spinor_gaussian(x[r * nb:], prec, 0, 40 + r)
+    flags = P.DSLASH_G5_IN | P.DSLASH_G5_OUT
+    first, count = lat.Vh // 3, lat.Vh - lat.Vh // 3 - 1
+    got = {}
+    for v in (2, 20, 21, 22):
+        _force(monkeypatch, v)
+        o = [dev_bytes(nb).fill_(7) for _ in range(5)]
+        lat.dslash(g, o[0], fe, 1, prec)
+        lat.dslash_xpay(g, o[1], fo, 0, prec, 0.25, x, -2.0, flags)
+        lat.dslash_full(g, o[2], o[3], fe, fo, prec)
+        lat.dslash_sites(g, o[4], fo, 0, prec, first, count, flags, 0.5, x, 1.5)
+        monkeypatch.setenv("PLQCD_MRHS_VARIANT", str(100 + v))
+        monkeypatch.setenv("PLQCD_MRHS_BLOCK", "64")
+        o.append(dev_bytes(n * nb))
+        lat.dslash_mrhs_xpay(g, o[5], fo, n, 0, prec, 0.25, x, -2.0, flags)
+        monkeypatch.delenv("PLQCD_MRHS_VARIANT")
+        lat.synchronize()
+        got[v] = o
+    for v in (20, 21, 22):
+        for k, (a, b) in enumerate(zip(got[v], got[2])):
+            assert bool((a == b).all()), (v, k)
+
+
+@pytest.mark.parametrize("dims", DIMS[1:])
+@pytest.mark.parametrize("variant", [20, 21])
+def test_ahead_f64_against_oracle(cuda, monkeypatch, restatement, dims, variant):
+    rng = np.random.default_rng(5)
+    V = O.volume(dims)
+    u, q = O.random_su3(4 * V, rng).reshape(4 * V, 9), O.gaussian_spinor(V, rng)
+    lat = new_lattice(dims)
+    g = P.Gauge(lat, P.F64, 18)
+    g.load_device(to_dev(u))
+    fe, fo = field_from_host(lat, q, 0, P.F64), field_from_host(lat, q, 1, P.F64)
+    oe, oo = dev_bytes(lat.spinor_bytes(P.F64)), dev_bytes(lat.spinor_bytes(P.F64))
+    _force(monkeypatch, variant)
+    lat.dslash_full(g, oe, oo, fe, fo, P.F64)
+    want = restatement.hop("eo", dims, q, u)
+    want = restatement.hop("oe", dims, q, u, want)
+    got = field_to_host(lat, oe, P.F64, 0) + field_to_host(lat, oo, P.F64, 1)
+    assert relmax(got, want) < 1e-14
