@@ -52,6 +52,35 @@ int lattice_workspace(plqcd_lattice *lat, size_t bytes, void **out) {
     return PLQCD_OK;
 }
 
+int lattice_staging(plqcd_lattice *lat, size_t bytes, void **out) {
+    if (bytes > kStagingBytes) return set_error(PLQCD_ERR_ARG, "staging of %zu bytes", bytes);
+    if (lat->staging_bytes < bytes) {
+        if (lat->staging) {
+            cudaStreamSynchronize(lat->stream);
+            cudaFree(lat->staging);
+            lat->staging = nullptr;
+            lat->staging_bytes = 0;
+        }
+        if (cudaMalloc(&lat->staging, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            return set_error(PLQCD_ERR_NOMEM, "staging of %zu bytes", bytes);
+        }
+        lat->staging_bytes = bytes;
+    }
+    *out = lat->staging;
+    return PLQCD_OK;
+}
+
+int lattice_host_block(plqcd_lattice *lat, void **out) {
+    if (!lat->host_block && cudaHostAlloc(&lat->host_block, kHostBlockBytes, cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        lat->host_block = nullptr;
+        return set_error(PLQCD_ERR_NOMEM, "page-locked block of %zu bytes", kHostBlockBytes);
+    }
+    *out = lat->host_block;
+    return PLQCD_OK;
+}
+
 }  // namespace plqcd
 
 namespace {
@@ -136,8 +165,9 @@ extern "C" int plqcd_invert_cg(plqcd_lattice *lat, const plqcd_gauge *g64, const
     void *redmem = take(red_scratch_bytes());
     PLQCD_CUDA_TRY(cudaMemsetAsync(redmem, 0, red_scratch_bytes(), s));
     RedScratch red = red_scratch_from(redmem);
-    CgState *hst = nullptr;
-    PLQCD_CUDA_TRY(cudaMallocHost(&hst, sizeof(CgState)));
+    void *hblock = nullptr;
+    PLQCD_TRY(lattice_host_block(lat, &hblock));
+    CgState *hst = static_cast<CgState *>(hblock);
     auto read_state = [&]() -> int {
         PLQCD_CUDA_TRY(cudaMemcpyAsync(hst, red.state, sizeof(CgState), cudaMemcpyDeviceToHost, s));
         PLQCD_CUDA_TRY(cudaStreamSynchronize(s));
@@ -297,7 +327,6 @@ extern "C" int plqcd_invert_cg(plqcd_lattice *lat, const plqcd_gauge *g64, const
     float ms = 0;
     cudaEventElapsedTime(&ms, e0, e1);
     inf.seconds = ms / 1e3;
-    cudaFreeHost(hst);
     // a hop whose staged loads never arrived leaves a flag, not a CUDA error
     if (!rc && dslash_tma_status(true))
         rc = set_error(PLQCD_ERR_TIMEOUT, "plqcd_invert_cg: a TMA stage wait of a hop ran out");

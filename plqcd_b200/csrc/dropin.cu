@@ -192,6 +192,21 @@ bool keep_cached_gauge(const void *u, const void *cached, bool dirty, uint64_t c
     return !dirty && cached == u && g_registered == u;
 }
 
+// A call queues the upload of its links and waits once, at its end. A call
+// that fails on the way waits as well (the caller gets its arrays back) and
+// marks the device copy of the links as not loaded.
+struct CallGuard {
+    bool &dirty;
+    bool ok = false;
+    ~CallGuard() {
+        if (ok) return;
+        for (cudaStream_t st : {g_d.s_h2d, g_d.s_d2h, g_d.stream})
+            if (st) cudaStreamSynchronize(st);
+        cudaGetLastError();
+        dirty = true;
+    }
+};
+
 int ensure_locked() {
     if (!plqcd_g.init) return set_error(PLQCD_ERR_STATE, "hopping matrix called before init_plqcd");
     const int *L = plqcd_g.latdims;
@@ -388,11 +403,12 @@ double hop_call(spinor *qin, spinor *qout, su3 *u, int out_parity) {
         return -1.0;
     }
     g_d.h2d = g_d.d2h = 0;
+    CallGuard guard{g_d.dirty};
 
     // gauge field: upload unless the device copy may serve (keep_cached_gauge)
     uint64_t fp = 0;
     if (!keep_cached_gauge(u, g_d.cached_u, g_d.dirty, g_d.fingerprint, &fp, [&] { return fingerprint(u, 8 * Vh); })) {
-        if (plqcd_gauge_load_host(g_d.gauge, u) != PLQCD_OK) return -1.0;
+        if (upload_links(g_d.gauge, u) != PLQCD_OK) return -1.0;
         g_d.cached_u = u;
         g_d.fingerprint = fp;
         g_d.dirty = false;
@@ -440,6 +456,7 @@ double hop_call(spinor *qin, spinor *qout, su3 *u, int out_parity) {
     }
     g_d.kernel_ms = kms;
     lat->last_kernel_ms = kms;
+    guard.ok = true;
     return stop_watch(t0);
 }
 
@@ -470,29 +487,19 @@ uint64_t fingerprint_split(const double *re, const double *im, long n) {
 int load_gauge_split(plqcd_gauge *g, const double *ure, const double *uim) {
     const Geom &geo = g->lat->geom;
     cudaStream_t s = g->lat->stream;
-    const long nlinks = 8 * geo.Vh, chunk = 1L << 20;
+    const long nlinks = 8 * geo.Vh, chunk = (long)(kStagingBytes / (18 * sizeof(double)));
     const long per = nlinks < chunk ? nlinks : chunk;
-    double *st = nullptr;
-    if (cudaMalloc(&st, sizeof(double) * 18 * per) != cudaSuccess) {
-        cudaGetLastError();
-        return set_error(PLQCD_ERR_NOMEM, "split gauge upload: staging allocation failed");
-    }
-    int rc = PLQCD_OK;
-    for (long first = 0; first < nlinks && rc == PLQCD_OK; first += per) {
+    std::lock_guard<std::mutex> lk(g->lat->staging_mu);
+    void *stage = nullptr;
+    PLQCD_TRY(lattice_staging(g->lat, sizeof(double) * 18 * per, &stage));
+    double *st = static_cast<double *>(stage);
+    for (long first = 0; first < nlinks; first += per) {
         const long n = nlinks - first < per ? nlinks - first : per;
-        cudaError_t e = cudaMemcpyAsync(st, ure + 9 * first, sizeof(double) * 9 * n, cudaMemcpyHostToDevice, s);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(st + 9 * per, uim + 9 * first, sizeof(double) * 9 * n, cudaMemcpyHostToDevice, s);
-        if (e != cudaSuccess) {
-            rc = set_error(PLQCD_ERR_CUDA, "split gauge upload: %s", cudaGetErrorString(e));
-            break;
-        }
-        rc = launch_gauge_import_split(geo, s, st, st + 9 * per, first, n, g->data, g->prec, g->recon);
-        if (rc == PLQCD_OK && cudaStreamSynchronize(s) != cudaSuccess)
-            rc = set_error(PLQCD_ERR_CUDA, "split gauge upload failed");
+        PLQCD_CUDA_TRY(cudaMemcpyAsync(st, ure + 9 * first, sizeof(double) * 9 * n, cudaMemcpyHostToDevice, s));
+        PLQCD_CUDA_TRY(cudaMemcpyAsync(st + 9 * per, uim + 9 * first, sizeof(double) * 9 * n, cudaMemcpyHostToDevice, s));
+        PLQCD_TRY(launch_gauge_import_split(geo, s, st, st + 9 * per, first, n, g->data, g->prec, g->recon));
     }
-    cudaFree(st);
-    return rc;
+    return PLQCD_OK;
 }
 
 double hop_call_split(double *qout_re, double *qout_im, double *u_re, double *u_im, double *qin_re,
@@ -514,6 +521,7 @@ double hop_call_split(double *qout_re, double *qout_im, double *u_re, double *u_
         return -1.0;
     }
     g_d.h2d = g_d.d2h = 0;
+    CallGuard guard{g_d.dirty_split};
     plqcd_gauge *&gf = short12 ? g_d.gauge12 : g_d.gauge_split;
     if (!gf && plqcd_gauge_create(lat, PLQCD_F64, short12 ? 12 : 18, &gf) != PLQCD_OK) return -1.0;
     SplitCache &sc = short12 ? g_d.split12 : g_d.split18;
@@ -564,6 +572,7 @@ double hop_call_split(double *qout_re, double *qout_im, double *u_re, double *u_
     cudaEventElapsedTime(&ms, g_d.ev_k0[0], g_d.ev_k1[0]);
     g_d.kernel_ms = ms;
     lat->last_kernel_ms = ms;
+    guard.ok = true;
     return stop_watch(t0);
 }
 
@@ -609,35 +618,24 @@ int relayout(cudaStream_t s, void *dst, const void *src, long nsites, int lanes,
     return PLQCD_OK;
 }
 
-// gauge field from a lane-packed host array, in chunks of sites
+// gauge field from a lane-packed host array, in chunks of whole packed objects
 int load_gauge_packed(plqcd_gauge *g, const void *u, int lanes) {
     const Geom &geo = g->lat->geom;
     cudaStream_t s = g->lat->stream;
-    const long nsites = 2 * geo.Vh, chunk = 1L << 18;  // sites per chunk (multiple of 4)
+    const long nsites = 2 * geo.Vh, chunk = (long)(kStagingBytes / (2 * 4 * sizeof(su3))) & ~3L;
     const long per = nsites < chunk ? nsites : chunk;
+    std::lock_guard<std::mutex> lk(g->lat->staging_mu);
     void *st = nullptr;
-    if (cudaMalloc(&st, 2 * per * 4 * sizeof(su3)) != cudaSuccess) {
-        cudaGetLastError();
-        return set_error(PLQCD_ERR_NOMEM, "packed gauge upload: staging allocation failed");
-    }
+    PLQCD_TRY(lattice_staging(g->lat, 2 * per * 4 * sizeof(su3), &st));
     char *packed = static_cast<char *>(st), *aos = packed + per * 4 * sizeof(su3);
-    int rc = PLQCD_OK;
-    for (long first = 0; first < nsites && rc == PLQCD_OK; first += per) {
+    for (long first = 0; first < nsites; first += per) {
         const long n = nsites - first < per ? nsites - first : per;
-        cudaError_t e = cudaMemcpyAsync(packed, static_cast<const char *>(u) + first * 4 * sizeof(su3),
-                                        n * 4 * sizeof(su3), cudaMemcpyHostToDevice, s);
-        if (e != cudaSuccess) {
-            rc = set_error(PLQCD_ERR_CUDA, "packed gauge upload: %s", cudaGetErrorString(e));
-            break;
-        }
-        rc = relayout(s, aos, packed, n, lanes, 36, true);
-        if (rc == PLQCD_OK)
-            rc = launch_gauge_import(geo, s, aos, 4 * first, 4 * n, g->data, g->prec, g->recon);
-        if (rc == PLQCD_OK && cudaStreamSynchronize(s) != cudaSuccess)
-            rc = set_error(PLQCD_ERR_CUDA, "packed gauge upload failed");
+        PLQCD_CUDA_TRY(cudaMemcpyAsync(packed, static_cast<const char *>(u) + first * 4 * sizeof(su3),
+                                       n * 4 * sizeof(su3), cudaMemcpyHostToDevice, s));
+        PLQCD_TRY(relayout(s, aos, packed, n, lanes, 36, true));
+        PLQCD_TRY(launch_gauge_import(geo, s, aos, 4 * first, 4 * n, g->data, g->prec, g->recon));
     }
-    cudaFree(st);
-    return rc;
+    return PLQCD_OK;
 }
 
 double hop_call_packed(const void *qin, void *qout, const void *u, int out_parity, int lanes, bool short12) {
@@ -662,6 +660,7 @@ double hop_call_packed(const void *qin, void *qout, const void *u, int out_parit
         return -1.0;
     }
     g_d.h2d = g_d.d2h = 0;
+    CallGuard guard{g_d.dirty_packed};
     plqcd_gauge *&gf = short12 ? g_d.gauge_packed12 : g_d.gauge_packed;
     if (!gf && plqcd_gauge_create(lat, PLQCD_F64, short12 ? 12 : 18, &gf) != PLQCD_OK) return -1.0;
     auto &pc = short12 ? g_d.packed12 : g_d.packed18;
@@ -711,6 +710,7 @@ double hop_call_packed(const void *qin, void *qout, const void *u, int out_parit
     cudaEventElapsedTime(&ms, g_d.ev_k0[0], g_d.ev_k1[0]);
     g_d.kernel_ms = ms;
     lat->last_kernel_ms = ms;
+    guard.ok = true;
     return stop_watch(t0);
 }
 

@@ -32,7 +32,7 @@
 namespace plqcd {
 
 int launch_dslash_ahead(cudaStream_t s, const dev::DslashArgs &a, int prec, int recon, bool xpay, bool full,
-                        int variant);
+                        bool joined, bool deep);
 
 namespace dev {
 
@@ -187,8 +187,8 @@ static int launch_pipe(const Geom &g, cudaStream_t s, const DslashArgs &a, int b
 }
 
 // variant 2, 3: cp.async pipeline of that depth; anything else: loads ahead
-// in registers (20, 21, 22 of dslash_ahead.cu; tuning files may still hold
-// 0, 12 and 13, kernels that it replaced)
+// in registers (0 and 21 of dslash_ahead.cu; tuning files may still hold 12
+// and 13, kernels that it replaced)
 template <class SIO, class LIO, bool COMPAT, bool XPAY, bool FULL>
 static int launch_t(const Geom &g, cudaStream_t s, const DslashArgs &a, int prec, int recon, int variant, int block) {
     if (variant == 2) return launch_pipe<SIO, LIO, 2, COMPAT, XPAY, FULL>(g, s, a, block);
@@ -199,7 +199,7 @@ static int launch_t(const Geom &g, cudaStream_t s, const DslashArgs &a, int prec
         PLQCD_CUDA_TRY(cudaGetLastError());
         return PLQCD_OK;
     } else {
-        return launch_dslash_ahead(s, a, prec, recon, XPAY, FULL, variant);
+        return launch_dslash_ahead(s, a, prec, recon, XPAY, FULL, variant == 21, block == 128);
     }
 }
 
@@ -258,14 +258,20 @@ int launch_dslash(const Geom &g, cudaStream_t s, const DslashCall &c) {
         int block = c.block > 0 ? c.block : (env_block > 0 ? env_block : 128);
         return dispatch(g, s, c, a, env_var >= 0 ? env_var : 2, block);
     }
-    char key[256];
     // a partial site range (the drop-in path's t-slab chunks) is a separate
     // entry: the TMA kernel takes whole fields only
     const bool part = a.h_begin != 0 || a.h_end != g.Vh;
+    const TuneId id = tune_id(kTuneDslash, c.prec, c.recon, c.full | (c.x ? 2 : 0) | (compat ? 4 : 0) | (part ? 8 : 0),
+                              c.nrhs, g.L);
+    TuneResult known;
+    if (tune_recall(id, &known)) return dispatch(g, s, c, a, known.variant, known.block);
+    char key[256];
     snprintf(key, sizeof key, "%sdslash|p%d|r%d|%s%s%s%s|%dx%dx%dx%d|n%d|c2", device_tag().c_str(), c.prec, c.recon,
              c.full ? "full" : "half", c.x ? "+xpay" : "", compat ? "+compat" : "", part ? "+range" : "", g.L[0],
              g.L[1], g.L[2], g.L[3], c.nrhs);
-    return tune_dslash(g, s, c, a, key);
+    const int rc = tune_dslash(g, s, c, a, key);
+    tune_remember(id, key);
+    return rc;
 }
 
 static int build_args(const Geom &g, const DslashCall &c, dev::DslashArgs &a) {
@@ -313,8 +319,9 @@ static int build_args(const Geom &g, const DslashCall &c, dev::DslashArgs &a) {
 
 static int tune_dslash(const Geom &g, cudaStream_t s, const DslashCall &c, const dev::DslashArgs &a,
                        const char *key) {
-    // loads ahead in registers (20, 21, 22), cp.async pipeline depth (2, 3)
-    // x block size. The first one runs where tuning is not possible.
+    // loads ahead in registers (0: a block of 64 stands for depth 1, one of
+    // 128 for depth 2; 21: joined parities), cp.async pipeline depth (2, 3) x
+    // block size. The first one runs where tuning is not possible.
     std::vector<TuneResult> cands;
     const bool compat = (c.flags & PLQCD_DSLASH_COMPAT) != 0;
     auto add = [&](int variant, int block) {
@@ -328,8 +335,8 @@ static int tune_dslash(const Geom &g, cudaStream_t s, const DslashCall &c, const
         add(0, 64);
     } else {
         if (c.full && c.prec == PLQCD_F64) add(21, 64);
-        if (c.prec != PLQCD_F64) add(22, 64);
-        add(20, 64);
+        if (c.prec != PLQCD_F64) add(0, 128);
+        add(0, 64);
         for (int v : {2, 3})
             for (int b : {64, 128, 256}) add(v, b);
     }

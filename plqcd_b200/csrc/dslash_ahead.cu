@@ -176,30 +176,29 @@ static int launch_ahead_m(cudaStream_t s, const DslashArgs &a, bool deep) {
 }
 
 template <int P, int RC>
-static int launch_ahead_pr(cudaStream_t s, const DslashArgs &a, bool xpay, bool full, int variant) {
+static int launch_ahead_pr(cudaStream_t s, const DslashArgs &a, bool xpay, bool full, bool joined, bool deep) {
     if (full) {
         if constexpr (P == PLQCD_F64)
-            if (variant == 21) return launch_ahead_m<P, RC, 3>(s, a, false);
-        return launch_ahead_m<P, RC, 2>(s, a, variant == 22);
+            if (joined) return launch_ahead_m<P, RC, 3>(s, a, false);
+        return launch_ahead_m<P, RC, 2>(s, a, deep);
     }
-    if (xpay) return launch_ahead_m<P, RC, 1>(s, a, variant == 22);
-    return launch_ahead_m<P, RC, 0>(s, a, variant == 22);
+    if (xpay) return launch_ahead_m<P, RC, 1>(s, a, deep);
+    return launch_ahead_m<P, RC, 0>(s, a, deep);
 }
 
 }  // namespace dev
 
-// variant 20: depth 1; 22: depth 2 (FP32-computing formats; depth 1 in
-// FP64); 21: full-lattice FP64 with joined parities in the tile order (any
-// other launch: as 20)
+// deep: depth 2 (the FP32-computing formats; FP64 always loads one ahead);
+// joined: mode 3 for the FP64 full lattice (without effect elsewhere)
 int launch_dslash_ahead(cudaStream_t s, const dev::DslashArgs &a, int prec, int recon, bool xpay, bool full,
-                        int variant) {
+                        bool joined, bool deep) {
     switch (prec * 100 + recon) {
-        case PLQCD_F64 * 100 + 18: return dev::launch_ahead_pr<PLQCD_F64, 18>(s, a, xpay, full, variant);
-        case PLQCD_F64 * 100 + 12: return dev::launch_ahead_pr<PLQCD_F64, 12>(s, a, xpay, full, variant);
-        case PLQCD_F32 * 100 + 18: return dev::launch_ahead_pr<PLQCD_F32, 18>(s, a, xpay, full, variant);
-        case PLQCD_F32 * 100 + 12: return dev::launch_ahead_pr<PLQCD_F32, 12>(s, a, xpay, full, variant);
-        case PLQCD_F16 * 100 + 12: return dev::launch_ahead_pr<PLQCD_F16, 12>(s, a, xpay, full, variant);
-        case PLQCD_BF16 * 100 + 12: return dev::launch_ahead_pr<PLQCD_BF16, 12>(s, a, xpay, full, variant);
+        case PLQCD_F64 * 100 + 18: return dev::launch_ahead_pr<PLQCD_F64, 18>(s, a, xpay, full, joined, deep);
+        case PLQCD_F64 * 100 + 12: return dev::launch_ahead_pr<PLQCD_F64, 12>(s, a, xpay, full, joined, deep);
+        case PLQCD_F32 * 100 + 18: return dev::launch_ahead_pr<PLQCD_F32, 18>(s, a, xpay, full, joined, deep);
+        case PLQCD_F32 * 100 + 12: return dev::launch_ahead_pr<PLQCD_F32, 12>(s, a, xpay, full, joined, deep);
+        case PLQCD_F16 * 100 + 12: return dev::launch_ahead_pr<PLQCD_F16, 12>(s, a, xpay, full, joined, deep);
+        case PLQCD_BF16 * 100 + 12: return dev::launch_ahead_pr<PLQCD_BF16, 12>(s, a, xpay, full, joined, deep);
         default:
             return set_error(PLQCD_ERR_ARG, "dslash: unsupported precision/reconstruction %d/%d", prec, recon);
     }

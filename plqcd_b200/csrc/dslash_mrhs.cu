@@ -822,6 +822,45 @@ int launch_dslash_mrhs(const Geom &g, cudaStream_t s, const void *gauge, int pre
     dev::MrhsArgs m;
     PLQCD_TRY(mrhs_args(g, gauge, prec, out, in, nrhs, out_parity, flags, a, x, b, m));
     const bool xpay = x != nullptr;
+    DslashCall dc;
+    dc.gauge = gauge;
+    dc.prec = prec;
+    dc.recon = recon;
+    dc.out = out;
+    dc.in = in;
+    dc.out_parity = out_parity;
+    dc.flags = flags;
+    dc.x = x;
+    dc.a_up = dc.a_low = a;
+    dc.b = b;
+    dc.nrhs = nrhs;
+    auto launch = [&](const TuneResult &t, char *dst) -> int {
+        if (t.variant >= 100000)
+            return launch_mrhs_tma(g, s, gauge, prec, recon, dst, in, nrhs, out_parity, flags, a, x, b, t.variant);
+        if (t.variant >= 3000 && t.variant < 4000)
+            return launch_dslash_mrhs_tc(g, s, gauge, prec, recon, dst, in, nrhs, out_parity, flags, a, x, b,
+                                         t.variant - 3000);
+        if (t.variant >= 100 && t.variant < 1000) {
+            DslashCall c2 = dc;
+            c2.out = dst;
+            return launch_dslash_config(g, s, c2, t.variant - 100, t.block);
+        }
+        dev::MrhsArgs tm = m;
+        tm.out = dst;
+        return mrhs_dispatch(g, s, prec, recon, tm, t.variant, t.block, xpay);
+    };
+    // explicit configuration for experiments and tests: bypasses the tuner
+    const char *ev = getenv("PLQCD_MRHS_VARIANT");
+    if (ev && *ev) {
+        const char *eb = getenv("PLQCD_MRHS_BLOCK");
+        TuneResult t;
+        t.variant = atoi(ev);
+        t.block = (eb && *eb) ? atoi(eb) : 128;
+        return launch(t, static_cast<char *>(out));
+    }
+    const TuneId id = tune_id(kTuneMrhs, prec, recon, xpay, nrhs, g.L);
+    TuneResult known;
+    if (tune_recall(id, &known)) return launch(known, static_cast<char *>(out));
     char key[256];
     mrhs_key(key, sizeof key, g, prec, recon, nrhs, xpay);
     // two families of candidates: the RHS-tile kernel above (variant = tile
@@ -890,53 +929,8 @@ int launch_dslash_mrhs(const Geom &g, cudaStream_t s, const void *gauge, int pre
             t.block = 128;
             cands.push_back(t);
         }
-    DslashCall dc;
-    dc.gauge = gauge;
-    dc.prec = prec;
-    dc.recon = recon;
-    dc.out = out;
-    dc.in = in;
-    dc.out_parity = out_parity;
-    dc.flags = flags;
-    dc.x = x;
-    dc.a_up = dc.a_low = a;
-    dc.b = b;
-    dc.nrhs = nrhs;
     void *scratch = nullptr;
-    // explicit configuration for experiments and tests: bypasses the tuner
-    const char *ev = getenv("PLQCD_MRHS_VARIANT");
-    if (ev && *ev) {
-        const char *eb = getenv("PLQCD_MRHS_BLOCK");
-        TuneResult t;
-        t.variant = atoi(ev);
-        t.block = (eb && *eb) ? atoi(eb) : 128;
-        if (t.variant >= 100 && t.variant < 1000) {
-            DslashCall c2 = dc;
-            return launch_dslash_config(g, s, c2, t.variant - 100, t.block);
-        }
-        if (t.variant >= 3000 && t.variant < 4000)
-            return launch_dslash_mrhs_tc(g, s, gauge, prec, recon, out, in, nrhs, out_parity, flags, a, x, b,
-                                         t.variant - 3000);
-        if (t.variant >= 100000)
-            return launch_mrhs_tma(g, s, gauge, prec, recon, out, in, nrhs, out_parity, flags, a, x, b, t.variant);
-        return mrhs_dispatch(g, s, prec, recon, m, t.variant, t.block, xpay);
-    }
     std::vector<int> tma_checked;
-    auto launch = [&](const TuneResult &t, char *dst) -> int {
-        if (t.variant >= 100000)
-            return launch_mrhs_tma(g, s, gauge, prec, recon, dst, in, nrhs, out_parity, flags, a, x, b, t.variant);
-        if (t.variant >= 3000 && t.variant < 4000)
-            return launch_dslash_mrhs_tc(g, s, gauge, prec, recon, dst, in, nrhs, out_parity, flags, a, x, b,
-                                         t.variant - 3000);
-        if (t.variant >= 100 && t.variant < 1000) {
-            DslashCall c2 = dc;
-            c2.out = dst;
-            return launch_dslash_config(g, s, c2, t.variant - 100, t.block);
-        }
-        dev::MrhsArgs tm = m;
-        tm.out = dst;
-        return mrhs_dispatch(g, s, prec, recon, tm, t.variant, t.block, xpay);
-    };
     auto run = [&](const TuneResult &t, bool trial) -> int {
         if (!trial) return launch(t, static_cast<char *>(out));
         if (!scratch && cudaMalloc(&scratch, m.fbytes * nrhs) != cudaSuccess) {
@@ -954,6 +948,7 @@ int launch_dslash_mrhs(const Geom &g, cudaStream_t s, const void *gauge, int pre
         return launch(t, static_cast<char *>(scratch));
     };
     int rc = tune_launch(key, s, cands, run);
+    tune_remember(id, key);
     if (scratch) {
         cudaStreamSynchronize(s);
         cudaFree(scratch);

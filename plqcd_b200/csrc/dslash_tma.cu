@@ -928,7 +928,7 @@ int launch_tma_t(cudaStream_t s, const dev::TmaMaps &m, const dev::TmaGeom &tg, 
                             : dev::k_dslash_tma_xy<SIO, LIO, XPAY, false>;
     PLQCD_TRY(smem_optin((const void *)k, smem));
     int occ = 0;
-    PLQCD_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, block, smem));
+    PLQCD_TRY(blocks_per_sm((const void *)k, block, smem, &occ));
     if (occ < 1) return set_error(PLQCD_ERR_ARG, "dslash: TMA tile does not fit on an SM (%zu B)", smem);
     long grid = (long)sm_count() * occ;
     if (grid > tg.nitems) grid = tg.nitems;

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <cstddef>
 #include <cstdint>
+#include <mutex>
 #include <string>
 
 #include "plqcd_b200.h"
@@ -71,6 +72,15 @@ struct plqcd_lattice {
     // solver workspace (grown on demand, released with the lattice)
     void *ws = nullptr;
     size_t ws_bytes = 0;
+    // kept between calls like the workspace, made on first use: device
+    // staging of host link arrays (at most kStagingBytes), a page-locked
+    // block for the scalars a solver reads back, the batched solver's stream
+    std::mutex staging_mu;  // held while an upload's copies and conversions are queued
+    void *staging = nullptr;
+    size_t staging_bytes = 0;
+    void *host_block = nullptr;
+    cudaStream_t solve_stream = nullptr;
+    cudaEvent_t solve_event = nullptr;
 };
 
 struct plqcd_gauge {
@@ -181,6 +191,10 @@ int launch_dslash_mrhs_sink(const Geom &g, cudaStream_t s, const void *gauge, in
 // once per (kernel, device) to at least `bytes` (utils.cpp)
 int smem_optin(const void *func, size_t bytes);
 
+// resident blocks per SM of kernel `func` on the current device, looked up
+// once per (kernel, device, block, bytes) (utils.cpp)
+int blocks_per_sm(const void *func, int block, size_t smem, int *out);
+
 // ID of the current CUDA context (unique within the process, never reused;
 // a cudaDeviceReset gives the device a new one), 0 when the driver does not
 // provide it (utils.cpp)
@@ -188,5 +202,15 @@ unsigned long long current_context_id();
 
 // device workspace of at least `bytes`, owned by the lattice (cg.cu)
 int lattice_workspace(plqcd_lattice *lat, size_t bytes, void **out);
+// the same for the upload staging; bytes <= kStagingBytes. Its use is
+// ordered by the lattice's stream, under staging_mu.
+constexpr size_t kStagingBytes = size_t(16) << 20;
+int lattice_staging(plqcd_lattice *lat, size_t bytes, void **out);
+// page-locked host block of kHostBlockBytes, owned by the lattice (cg.cu)
+constexpr size_t kHostBlockBytes = 4096;
+int lattice_host_block(plqcd_lattice *lat, void **out);
+// links in the API layout on the host -> gauge field, through the staging;
+// the copies are ordered on the lattice's stream and not waited for (api.cu)
+int upload_links(plqcd_gauge *g, const su3 *u_host);
 
 }  // namespace plqcd

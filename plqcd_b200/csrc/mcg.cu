@@ -605,7 +605,7 @@ struct Batch {
 // item takes its lattice's solver workspace, kept across solves as
 // plqcd_invert_cg keeps it, unless an earlier item of the batch holds it:
 // then it allocates its own (`it.mem`, freed after the solve).
-int alloc_item(Batch &B, Item &it, bool own_ws) {
+int alloc_item(Batch &B, Item &it, bool own_ws, int nitems) {
     const plqcd_solve_item &in = it.in;
     it.g = &in.lat->geom;
     const long Vh = it.g->Vh;
@@ -619,7 +619,7 @@ int alloc_item(Batch &B, Item &it, bool own_ws) {
     const size_t nsb = (size_t)(Vh + 31) / 32;  // site blocks of a fused hop, at most
     const size_t need = 4 * al(it.fb64 * n) + 5 * al(it.fbs * n) + al(it.fbx * n) + 10 * al(sizeof(double) * n) +
                         3 * al(sizeof(int) * n) + al(sizeof(double) * n * it.st.nb) + al(sizeof(unsigned) * n) +
-                        al(sizeof(double) * n * nsb);
+                        al(sizeof(double) * n * nsb) + al(sizeof(McgControl)) + al(sizeof(McgState) * nitems);
     void *ws = nullptr;
     if (own_ws) {
         if (cudaMalloc(&it.mem, need) != cudaSuccess) {
@@ -655,6 +655,9 @@ int alloc_item(Batch &B, Item &it, bool own_ws) {
     it.st.partials = reinterpret_cast<double *>(take(sizeof(double) * n * it.st.nb));
     it.st.counters = reinterpret_cast<unsigned *>(take(sizeof(unsigned) * n));
     it.hop_partials = reinterpret_cast<double *>(take(sizeof(double) * n * nsb));
+    // the first item's workspace also holds the batch's control block and states
+    if (!B.ctl) B.ctl = reinterpret_cast<McgControl *>(take(sizeof(McgControl)));
+    if (!B.st_dev) B.st_dev = reinterpret_cast<McgState *>(take(sizeof(McgState) * nitems));
     cudaStream_t s = B.s;
     PLQCD_CUDA_TRY(cudaMemsetAsync(it.st.counters, 0, sizeof(unsigned) * n, s));
     PLQCD_CUDA_TRY(cudaMemsetAsync(it.st.conv_iter, 0xff, sizeof(int) * n, s));
@@ -882,39 +885,31 @@ extern "C" int plqcd_invert_cg_batch(plqcd_solve_item *items, int nitems, const 
     B.tol = prm->tol;
     B.delta = prm->delta;
     B.mixed = prm->sloppy_prec != PLQCD_F64;
-    // the batch runs on a private stream ordered after the first lattice's
-    // stream (graph capture cannot use the legacy default stream)
-    cudaStream_t user = items[0].lat->stream;
-    PLQCD_CUDA_TRY(cudaStreamCreateWithFlags(&B.s, cudaStreamNonBlocking));
-    cudaEvent_t ev0, ev1, evu;
-    cudaEventCreate(&ev0);
-    cudaEventCreate(&ev1);
-    cudaEventCreateWithFlags(&evu, cudaEventDisableTiming);
-    cudaEventRecord(evu, user);
-    cudaStreamWaitEvent(B.s, evu, 0);
+    // the batch runs on a stream of its own, ordered after the first
+    // lattice's stream (graph capture cannot use the legacy default stream);
+    // that lattice keeps the stream, its events and the page-locked block
+    // between calls: making them on every call cost 3 to 30 ms
+    plqcd_lattice *owner = items[0].lat;
+    cudaStream_t user = owner->stream;
+    void *hblock = nullptr;
+    PLQCD_TRY(lattice_host_block(owner, &hblock));
+    static_assert(sizeof(McgControl) <= kHostBlockBytes, "control block");
+    if (!owner->solve_stream)
+        PLQCD_CUDA_TRY(cudaStreamCreateWithFlags(&owner->solve_stream, cudaStreamNonBlocking));
+    if (!owner->solve_event)
+        PLQCD_CUDA_TRY(cudaEventCreateWithFlags(&owner->solve_event, cudaEventDisableTiming));
+    B.s = owner->solve_stream;
+    cudaEvent_t ev0 = owner->ev0, ev1 = owner->ev1, evu = owner->solve_event;
+    PLQCD_CUDA_TRY(cudaEventRecord(evu, user));
+    PLQCD_CUDA_TRY(cudaStreamWaitEvent(B.s, evu, 0));
 
     int rc = PLQCD_OK;
-    McgControl *hctl = nullptr;
+    McgControl *hctl = static_cast<McgControl *>(hblock);
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t gexec = nullptr;
     plqcd_batch_info inf;
     memset(&inf, 0, sizeof inf);
     do {
-        if (cudaMalloc(&B.ctl, sizeof(McgControl)) != cudaSuccess ||
-            cudaMalloc(&B.st_dev, sizeof(McgState) * nitems) != cudaSuccess ||
-            cudaMallocHost(&hctl, sizeof(McgControl)) != cudaSuccess) {
-            cudaGetLastError();
-            rc = set_error(PLQCD_ERR_NOMEM, "plqcd_invert_cg_batch: control allocation");
-            break;
-        }
-        McgControl c0{};
-        c0.max_iter = prm->max_iter;
-        c0.tol2 = prm->tol * prm->tol;
-        c0.delta2 = prm->delta * prm->delta;
-        if ((rc = cudaMemcpyAsync(B.ctl, &c0, sizeof c0, cudaMemcpyHostToDevice, B.s) == cudaSuccess
-                      ? PLQCD_OK
-                      : set_error(PLQCD_ERR_CUDA, "plqcd_invert_cg_batch: control upload")))
-            break;
         // outside the timed solve: workspaces, tuning of every hop the loop
         // launches, and the graph (capture and instantiation run nothing)
         B.items.resize(nitems);
@@ -925,7 +920,17 @@ extern "C" int plqcd_invert_cg_batch(plqcd_solve_item *items, int nitems, const 
             it.xprec = (it.ps == PLQCD_F64) ? PLQCD_F64 : PLQCD_F32;
             bool shared = false;
             for (int j = 0; j < k; j++) shared = shared || items[j].lat == items[k].lat;
-            rc = alloc_item(B, it, shared);
+            rc = alloc_item(B, it, shared, nitems);
+        }
+        if (rc) break;
+        McgControl c0{};
+        c0.max_iter = prm->max_iter;
+        c0.tol2 = prm->tol * prm->tol;
+        c0.delta2 = prm->delta * prm->delta;
+        *hctl = c0;
+        if (cudaMemcpyAsync(B.ctl, hctl, sizeof c0, cudaMemcpyHostToDevice, B.s) != cudaSuccess) {
+            rc = set_error(PLQCD_ERR_CUDA, "plqcd_invert_cg_batch: control upload");
+            break;
         }
         for (int k = 0; k < nitems && rc == PLQCD_OK; k++) rc = tune_item(B, B.items[k]);
         if (rc) break;
@@ -1007,15 +1012,8 @@ extern "C" int plqcd_invert_cg_batch(plqcd_solve_item *items, int nitems, const 
     if (graph) cudaGraphDestroy(graph);
     for (Item &it : B.items)
         if (it.mem) cudaFree(it.mem);
-    if (B.ctl) cudaFree(B.ctl);
-    if (B.st_dev) cudaFree(B.st_dev);
-    if (hctl) cudaFreeHost(hctl);
-    cudaEventDestroy(ev0);
-    cudaEventDestroy(ev1);
     cudaEventRecord(evu, B.s);
     cudaStreamWaitEvent(user, evu, 0);
-    cudaEventDestroy(evu);
-    cudaStreamDestroy(B.s);
     if (info) *info = inf;
     if (rc) return rc;
     if (!inf.converged) return set_error(PLQCD_ERR_NOCONV, "plqcd_invert_cg_batch: not converged in %d iterations", inf.iterations);

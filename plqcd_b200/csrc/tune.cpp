@@ -23,6 +23,7 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <unordered_map>
 
 #include "internal.h"
 #include "tune.h"
@@ -35,6 +36,17 @@ std::mutex g_mu;
 std::map<std::string, TuneResult> &cache() {
     static std::map<std::string, TuneResult> c;
     return c;
+}
+struct TuneIdHash {
+    size_t operator()(const TuneId &id) const {
+        uint64_t h = 1469598103934665603ULL;
+        for (int x : id.v) h = (h ^ (uint32_t)x) * 1099511628211ULL;
+        return (size_t)h;
+    }
+};
+std::unordered_map<TuneId, TuneResult, TuneIdHash> &known() {
+    static std::unordered_map<TuneId, TuneResult, TuneIdHash> k;
+    return k;
 }
 bool g_loaded = false;
 int g_enabled = -1;
@@ -257,6 +269,28 @@ bool tune_lookup(const std::string &key, TuneResult *out) {
     return find_locked(key, !tune_enabled(), out);
 }
 
+bool TuneId::operator==(const TuneId &o) const { return memcmp(v, o.v, sizeof v) == 0; }
+
+TuneId tune_id(TuneFamily family, int prec, int recon, int mode, int nrhs, const int dims[4]) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    return TuneId{{dev, family, prec, recon, mode, nrhs, dims[0], dims[1], dims[2], dims[3], 0, 0}};
+}
+
+bool tune_recall(const TuneId &id, TuneResult *out) {
+    std::lock_guard<std::mutex> lk(g_mu);
+    auto it = known().find(id);
+    if (it == known().end()) return false;
+    *out = it->second;
+    return true;
+}
+
+void tune_remember(const TuneId &id, const std::string &key) {
+    std::lock_guard<std::mutex> lk(g_mu);
+    TuneResult r;
+    if (find_locked(key, false, &r)) known()[id] = r;
+}
+
 }  // namespace plqcd
 
 extern "C" int plqcd_tune_enable(int on) {
@@ -267,6 +301,7 @@ extern "C" int plqcd_tune_enable(int on) {
 extern "C" int plqcd_tune_clear(void) {
     std::lock_guard<std::mutex> lk(plqcd::g_mu);
     plqcd::cache().clear();
+    plqcd::known().clear();
     plqcd::g_loaded = true;  // do not reload the file
     return PLQCD_OK;
 }
@@ -280,6 +315,7 @@ extern "C" int plqcd_tune_save(const char *path) {
 extern "C" int plqcd_tune_load(const char *path) {
     std::lock_guard<std::mutex> lk(plqcd::g_mu);
     plqcd::load_locked(path ? path : plqcd::default_path());
+    plqcd::known().clear();
     plqcd::g_loaded = true;
     return PLQCD_OK;
 }

@@ -25,4 +25,20 @@ int tune_launch(const std::string &key, cudaStream_t s, const std::vector<TuneRe
 const std::string &device_tag();
 bool tune_lookup(const std::string &key, TuneResult *out);
 
+// What tells the launches of the tuned families apart, as numbers: the look-up
+// of a launch that is already tuned needs no key text and no candidate list
+// (a hop of a 4x6x8x10 lattice runs 4 us on the device; building them took
+// 2 us, 18 with the tile plans of the TMA candidates).
+struct TuneId {
+    int v[12];  // device, family, precision, reconstruction, mode bits, RHS, extents (the rest 0)
+    bool operator==(const TuneId &o) const;
+};
+enum TuneFamily : int { kTuneDslash = 1, kTuneMrhs = 2 };
+TuneId tune_id(TuneFamily family, int prec, int recon, int mode, int nrhs, const int dims[4]);
+// the tuned configuration of `id`, once tune_remember has tied it to the
+// entry of `key` (no effect while there is no such entry); dropped when
+// entries are cleared or loaded
+bool tune_recall(const TuneId &id, TuneResult *out);
+void tune_remember(const TuneId &id, const std::string &key);
+
 }  // namespace plqcd

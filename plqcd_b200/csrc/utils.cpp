@@ -15,6 +15,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <map>
+#include <tuple>
 #include <mutex>
 #include <thread>
 #include <unordered_map>
@@ -178,6 +179,22 @@ int smem_optin(const void *func, size_t bytes) {
         return set_error(PLQCD_ERR_CUDA, "shared-memory opt-in of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
     }
     have = bytes;
+    return PLQCD_OK;
+}
+
+int blocks_per_sm(const void *func, int block, size_t smem, int *out) {
+    static std::mutex mu;
+    static std::map<std::tuple<const void *, int, int, size_t>, int> seen;
+    int dev = 0;
+    PLQCD_CUDA_TRY(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lk(mu);
+    auto it = seen.find({func, dev, block, smem});
+    if (it != seen.end()) {
+        *out = it->second;
+        return PLQCD_OK;
+    }
+    PLQCD_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(out, func, block, smem));
+    seen[{func, dev, block, smem}] = *out;
     return PLQCD_OK;
 }
 

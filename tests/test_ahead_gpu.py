@@ -16,9 +16,13 @@ FORMATS = [(P.F64, 18), (P.F64, 12), (P.F32, 18), (P.F32, 12), (P.F16, 12), (P.B
 DIMS = [(2, 2, 2, 2), (10, 6, 2, 2), (6, 10, 14, 2), (12, 4, 6, 10)]
 
 
-def _force(monkeypatch, variant):
+# (variant, block): depth 1, depth 2, joined parities (full-lattice FP64)
+CONFIGS = [(0, 64), (0, 128), (21, 64)]
+
+
+def _force(monkeypatch, variant, block):
     monkeypatch.setenv("PLQCD_DSLASH_STAGES", str(variant))
-    monkeypatch.setenv("PLQCD_DSLASH_BLOCK", "64")
+    monkeypatch.setenv("PLQCD_DSLASH_BLOCK", str(block))
 
 
 @pytest.mark.parametrize("dims", DIMS)
@@ -37,28 +41,28 @@ def test_ahead_same_bits(cuda, monkeypatch, dims, prec, recon):
     flags = P.DSLASH_G5_IN | P.DSLASH_G5_OUT
     first, count = lat.Vh // 3, lat.Vh - lat.Vh // 3 - 1
     got = {}
-    for v in (2, 20, 21, 22):
-        _force(monkeypatch, v)
+    for v in [(2, 64)] + CONFIGS:
+        _force(monkeypatch, *v)
         o = [dev_bytes(nb).fill_(7) for _ in range(5)]
         lat.dslash(g, o[0], fe, 1, prec)
         lat.dslash_xpay(g, o[1], fo, 0, prec, 0.25, x, -2.0, flags)
         lat.dslash_full(g, o[2], o[3], fe, fo, prec)
         lat.dslash_sites(g, o[4], fo, 0, prec, first, count, flags, 0.5, x, 1.5)
-        monkeypatch.setenv("PLQCD_MRHS_VARIANT", str(100 + v))
-        monkeypatch.setenv("PLQCD_MRHS_BLOCK", "64")
+        monkeypatch.setenv("PLQCD_MRHS_VARIANT", str(100 + v[0]))
+        monkeypatch.setenv("PLQCD_MRHS_BLOCK", str(v[1]))
         o.append(dev_bytes(n * nb))
         lat.dslash_mrhs_xpay(g, o[5], fo, n, 0, prec, 0.25, x, -2.0, flags)
         monkeypatch.delenv("PLQCD_MRHS_VARIANT")
         lat.synchronize()
         got[v] = o
-    for v in (20, 21, 22):
-        for k, (a, b) in enumerate(zip(got[v], got[2])):
+    for v in CONFIGS:
+        for k, (a, b) in enumerate(zip(got[v], got[2, 64])):
             assert bool((a == b).all()), (v, k)
 
 
 @pytest.mark.parametrize("dims", DIMS[1:])
-@pytest.mark.parametrize("variant", [20, 21])
-def test_ahead_f64_against_oracle(cuda, monkeypatch, restatement, dims, variant):
+@pytest.mark.parametrize("config", [(0, 64), (21, 64)])
+def test_ahead_f64_against_oracle(cuda, monkeypatch, restatement, dims, config):
     rng = np.random.default_rng(5)
     V = O.volume(dims)
     u, q = O.random_su3(4 * V, rng).reshape(4 * V, 9), O.gaussian_spinor(V, rng)
@@ -67,7 +71,7 @@ def test_ahead_f64_against_oracle(cuda, monkeypatch, restatement, dims, variant)
     g.load_device(to_dev(u))
     fe, fo = field_from_host(lat, q, 0, P.F64), field_from_host(lat, q, 1, P.F64)
     oe, oo = dev_bytes(lat.spinor_bytes(P.F64)), dev_bytes(lat.spinor_bytes(P.F64))
-    _force(monkeypatch, variant)
+    _force(monkeypatch, *config)
     lat.dslash_full(g, oe, oo, fe, fo, P.F64)
     want = restatement.hop("eo", dims, q, u)
     want = restatement.hop("oe", dims, q, u, want)
