@@ -66,7 +66,8 @@ extern "C" int plqcd_lattice_destroy(plqcd_lattice *lat) {
     if (lat->staging) cudaFree(lat->staging);
     if (lat->host_block) cudaFreeHost(lat->host_block);
     if (lat->solve_stream) cudaStreamDestroy(lat->solve_stream);
-    if (lat->solve_event) cudaEventDestroy(lat->solve_event);
+    for (cudaEvent_t ev : {lat->solve_event, lat->iter_event[0], lat->iter_event[1]})
+        if (ev) cudaEventDestroy(ev);
     if (lat->ev0) cudaEventDestroy(lat->ev0);
     if (lat->ev1) cudaEventDestroy(lat->ev1);
     delete lat;

@@ -1,9 +1,10 @@
 // blas.cu -- vector kernels and deterministic FP64 reductions.
 //
-// Reductions accumulate in FP64 whatever the storage precision. Each block
-// writes its partial sum; the last block to arrive (atomic ticket) adds the
-// partials in a fixed order, so results do not depend on block scheduling,
-// and applies the solver-scalar update selected by RedOp.
+// The batched norm accumulates in FP64 whatever the storage precision. Each
+// block writes its partial sum; the last block to arrive (atomic ticket) adds
+// the partials in a fixed order, so results do not depend on block
+// scheduling. (The sums of the single-RHS solver are in the epilogues of its
+// hops, dslash_ahead.cu.)
 #include <cuda_runtime.h>
 
 #include "blas.cuh"
@@ -11,14 +12,20 @@
 
 namespace plqcd {
 
-size_t red_scratch_bytes() { return sizeof(double) * kMaxRedBlocks * 2 + 256 + sizeof(CgState); }
+static size_t red_partials(long Vh) {
+    const size_t n = hop_sum_partials(Vh);
+    return n > (size_t)kMaxRedBlocks ? n : (size_t)kMaxRedBlocks;
+}
 
-RedScratch red_scratch_from(void *mem) {
+size_t red_scratch_bytes(long Vh) { return sizeof(double) * red_partials(Vh) + 256 + sizeof(CgState); }
+
+RedScratch red_scratch_from(void *mem, long Vh) {
     RedScratch r;
     char *p = static_cast<char *>(mem);
+    const size_t n = sizeof(double) * red_partials(Vh);
     r.partials = reinterpret_cast<double *>(p);
-    r.counter = reinterpret_cast<unsigned *>(p + sizeof(double) * kMaxRedBlocks * 2);
-    r.state = reinterpret_cast<CgState *>(p + sizeof(double) * kMaxRedBlocks * 2 + 256);
+    r.counter = reinterpret_cast<unsigned *>(p + n);
+    r.state = reinterpret_cast<CgState *>(p + n + 256);
     return r;
 }
 
@@ -29,66 +36,6 @@ inline int blas_grid(long n) {
     return (int)(b < kMaxRedBlocks ? b : kMaxRedBlocks);
 }
 
-__device__ __forceinline__ void apply_op(RedOp op, double sum, CgState *st) {
-    switch (op) {
-        case RED_AUX: st->aux = sum; break;
-        case RED_ALPHA:
-            st->pAp = sum;
-            st->alpha = sum > 0 ? st->rr / sum : 0.0;
-            break;
-        case RED_RR:
-            st->rr_old = st->rr;
-            st->rr = sum;
-            st->beta = st->rr_old > 0 ? sum / st->rr_old : 0.0;
-            break;
-        case RED_SR2: st->sr2 = sum; break;
-        case RED_RR_TRUE:
-            st->rr = sum;
-            st->beta = st->rr_old > 0 ? sum / st->rr_old : 0.0;
-            break;
-        case RED_RR_INIT:
-            st->rr = sum;
-            st->rr_old = sum;
-            break;
-    }
-}
-
-// Block-reduce v, publish the partial, and let the last block finish.
-__device__ void reduce_finish(double v, RedScratch r, RedOp op) {
-    __shared__ double warp_sums[kBlasBlock / 32];
-    __shared__ bool last;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (lane == 0) warp_sums[w] = v;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double b = 0;
-        for (int k = 0; k < (int)(blockDim.x >> 5); k++) b += warp_sums[k];
-        r.partials[blockIdx.x] = b;
-        __threadfence();
-        unsigned ticket = atomicAdd(r.counter, 1u);
-        last = (ticket == gridDim.x - 1);
-    }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    // fixed-order sum of the partials
-    double t = 0;
-    for (int k = threadIdx.x; k < (int)gridDim.x; k += blockDim.x) t += ((volatile double *)r.partials)[k];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    __syncthreads();
-    if (lane == 0) warp_sums[w] = t;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double tot = 0;
-        for (int k = 0; k < (int)(blockDim.x >> 5); k++) tot += warp_sums[k];
-        apply_op(op, tot, r.state);
-        *r.counter = 0;  // ready for the next reduction on this scratch
-    }
-}
-
 template <typename R>
 __device__ __forceinline__ double norm2_site(const cx<R> v[12]) {
     double s = 0;
@@ -97,57 +44,13 @@ __device__ __forceinline__ double norm2_site(const cx<R> v[12]) {
     return s;
 }
 
-template <int P>
-__global__ void __launch_bounds__(kBlasBlock) k_norm2(const void *x, long Vh, RedScratch r, RedOp op) {
-    using R = typename SpinorIO<P>::real;
-    double acc = 0;
-    for (long h = (long)blockIdx.x * blockDim.x + threadIdx.x; h < Vh; h += (long)gridDim.x * blockDim.x) {
-        cx<R> v[12];
-        SpinorIO<P>::load(x, Vh, h, v);
-        acc += norm2_site(v);
-    }
-    reduce_finish(acc, r, op);
-}
-
-__global__ void __launch_bounds__(kBlasBlock) k_sub_norm2(void *out, const void *a, const void *b, long Vh,
-                                                          RedScratch r, RedOp op) {
-    double acc = 0;
-    for (long h = (long)blockIdx.x * blockDim.x + threadIdx.x; h < Vh; h += (long)gridDim.x * blockDim.x) {
-        cx<double> av[12], bv[12];
-        SpinorIO<PLQCD_F64>::load(a, Vh, h, av);
-        SpinorIO<PLQCD_F64>::load(b, Vh, h, bv);
-#pragma unroll
-        for (int k = 0; k < 12; k++) av[k] = csub(av[k], bv[k]);
-        SpinorIO<PLQCD_F64>::store(out, Vh, h, av);
-        acc += norm2_site(av);
-    }
-    reduce_finish(acc, r, op);
-}
-
-// r_s -= alpha Ap ; |r_s|^2 (the solution update of the iteration is in k_cg_p_x)
-template <int P>
-__global__ void __launch_bounds__(kBlasBlock) k_cg_update_r(void *rs, const void *Ap, long Vh, RedScratch r) {
-    using R = typename SpinorIO<P>::real;
-    const R a = (R)r.state->alpha;
-    double acc = 0;
-    for (long h = (long)blockIdx.x * blockDim.x + threadIdx.x; h < Vh; h += (long)gridDim.x * blockDim.x) {
-        cx<R> av[12], rv[12];
-        SpinorIO<P>::load(Ap, Vh, h, av);
-        SpinorIO<P>::load(rs, Vh, h, rv);
-#pragma unroll
-        for (int k = 0; k < 12; k++) rv[k] = {fma(-a, av[k].re, rv[k].re), fma(-a, av[k].im, rv[k].im)};
-        SpinorIO<P>::store(rs, Vh, h, rv);
-        acc += norm2_site(rv);
-    }
-    reduce_finish(acc, r, RED_RR);
-}
-
 // XMODE 1: x_s = alpha p (x_s counts as zero); 2: x_s += alpha p; 0: no x
 // update (a reliable update folded alpha p into x). Then p = r + beta p.
 template <int P, int XP, int XMODE>
 __global__ void __launch_bounds__(kBlasBlock) k_cg_p_x(void *p, const void *rs, void *xs, long Vh, const CgState *st) {
     using R = typename SpinorIO<P>::real;
     using RX = typename SpinorIO<XP>::real;
+    if (XMODE && st->halt) return;
     const R beta = (R)st->beta;
     const RX ax = (RX)st->alpha;
     for (long h = (long)blockIdx.x * blockDim.x + threadIdx.x; h < Vh; h += (long)gridDim.x * blockDim.x) {
@@ -204,39 +107,6 @@ __global__ void __launch_bounds__(kBlasBlock) k_accum(void *x64, const void *xs,
     }
 }
 
-// z = a - b (F64) ; |z|^2 -> op ; out = z in format SP (z itself is not stored)
-template <int SP>
-__global__ void __launch_bounds__(kBlasBlock) k_sub_norm2_to(void *out, const void *a, const void *b, long Vh,
-                                                             RedScratch r, RedOp op) {
-    using RS = typename SpinorIO<SP>::real;
-    double acc = 0;
-    for (long h = (long)blockIdx.x * blockDim.x + threadIdx.x; h < Vh; h += (long)gridDim.x * blockDim.x) {
-        cx<double> av[12], bv[12];
-        SpinorIO<PLQCD_F64>::load(a, Vh, h, av);
-        SpinorIO<PLQCD_F64>::load(b, Vh, h, bv);
-        cx<RS> d[12];
-#pragma unroll
-        for (int k = 0; k < 12; k++) {
-            av[k] = csub(av[k], bv[k]);
-            d[k] = {(RS)av[k].re, (RS)av[k].im};
-        }
-        SpinorIO<SP>::store(out, Vh, h, d);
-        acc += norm2_site(av);
-    }
-    reduce_finish(acc, r, op);
-}
-
-__global__ void __launch_bounds__(kBlasBlock) k_axpby64(double a, const void *x, double b, void *y, long Vh) {
-    for (long h = (long)blockIdx.x * blockDim.x + threadIdx.x; h < Vh; h += (long)gridDim.x * blockDim.x) {
-        cx<double> xv[12], yv[12];
-        SpinorIO<PLQCD_F64>::load(x, Vh, h, xv);
-        SpinorIO<PLQCD_F64>::load(y, Vh, h, yv);
-#pragma unroll
-        for (int k = 0; k < 12; k++) yv[k] = {fma(a, xv[k].re, b * yv[k].re), fma(a, xv[k].im, b * yv[k].im)};
-        SpinorIO<PLQCD_F64>::store(y, Vh, h, yv);
-    }
-}
-
 }  // namespace dev
 
 #define BLAS_PREC_SWITCH(prec, F)                                                   \
@@ -247,31 +117,6 @@ __global__ void __launch_bounds__(kBlasBlock) k_axpby64(double a, const void *x,
         case PLQCD_BF16: F(PLQCD_BF16); break;                                      \
         default: return set_error(PLQCD_ERR_ARG, "blas: unknown precision %d", prec); \
     }
-
-int blas_norm2(const Geom &g, cudaStream_t s, const void *x, int prec, const RedScratch &r, RedOp op) {
-    const int nb = dev::blas_grid(g.Vh);
-#define F(P) dev::k_norm2<P><<<nb, kBlasBlock, 0, s>>>(x, g.Vh, r, op)
-    BLAS_PREC_SWITCH(prec, F)
-#undef F
-    PLQCD_CUDA_TRY(cudaGetLastError());
-    return PLQCD_OK;
-}
-
-int blas_sub_norm2(const Geom &g, cudaStream_t s, void *out, const void *a, const void *b, const RedScratch &r,
-                   RedOp op) {
-    dev::k_sub_norm2<<<dev::blas_grid(g.Vh), kBlasBlock, 0, s>>>(out, a, b, g.Vh, r, op);
-    PLQCD_CUDA_TRY(cudaGetLastError());
-    return PLQCD_OK;
-}
-
-int blas_cg_update_r(const Geom &g, cudaStream_t s, void *rs, const void *Ap, int prec, const RedScratch &r) {
-    const int nb = dev::blas_grid(g.Vh);
-#define F(P) dev::k_cg_update_r<P><<<nb, kBlasBlock, 0, s>>>(rs, Ap, g.Vh, r)
-    BLAS_PREC_SWITCH(prec, F)
-#undef F
-    PLQCD_CUDA_TRY(cudaGetLastError());
-    return PLQCD_OK;
-}
 
 int blas_cg_p_x(const Geom &g, cudaStream_t s, void *p, const void *rs, int prec, void *xs, int xprec, int xmode,
                 const RedScratch &r) {
@@ -324,22 +169,6 @@ int blas_accum(const Geom &g, cudaStream_t s, void *x64, const void *xs, int xpr
 #undef F
 #undef G
     }
-    PLQCD_CUDA_TRY(cudaGetLastError());
-    return PLQCD_OK;
-}
-
-int blas_sub_norm2_to(const Geom &g, cudaStream_t s, void *out, int prec, const void *a, const void *b,
-                      const RedScratch &r, RedOp op) {
-    const int nb = dev::blas_grid(g.Vh);
-#define F(P) dev::k_sub_norm2_to<P><<<nb, kBlasBlock, 0, s>>>(out, a, b, g.Vh, r, op)
-    BLAS_PREC_SWITCH(prec, F)
-#undef F
-    PLQCD_CUDA_TRY(cudaGetLastError());
-    return PLQCD_OK;
-}
-
-int blas_axpby64(const Geom &g, cudaStream_t s, double a, const void *x, double b, void *y) {
-    dev::k_axpby64<<<dev::blas_grid(g.Vh), kBlasBlock, 0, s>>>(a, x, b, y, g.Vh);
     PLQCD_CUDA_TRY(cudaGetLastError());
     return PLQCD_OK;
 }

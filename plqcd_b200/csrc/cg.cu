@@ -89,9 +89,9 @@ struct Op {
     const Geom &g;
     cudaStream_t s;
     double kappa;
-    // out_parity-specific hopping with epilogue
-    int hop(const plqcd_gauge *gf, void *out, const void *in, int out_parity, unsigned flags, const void *x = nullptr,
-            double a = 1.0, double b = 0.0) const {
+    const RedScratch &red;
+    static DslashCall call(const plqcd_gauge *gf, void *out, const void *in, int out_parity, unsigned flags,
+                           const void *x, double a, double b, const int *halt) {
         DslashCall c;
         c.gauge = gf->data;
         c.prec = gf->prec;
@@ -103,7 +103,13 @@ struct Op {
         c.x = x;
         c.a_up = c.a_low = a;
         c.b = b;
-        return launch_dslash(g, s, c);
+        c.halt = halt;
+        return c;
+    }
+    // out_parity-specific hopping with epilogue
+    int hop(const plqcd_gauge *gf, void *out, const void *in, int out_parity, unsigned flags, const void *x = nullptr,
+            double a = 1.0, double b = 0.0, const int *halt = nullptr) const {
+        return launch_dslash(g, s, call(gf, out, in, out_parity, flags, x, a, b, halt));
     }
     // out = Mhat in (dagger: g5 Mhat g5 in); tmp_o: odd scratch
     int mhat(const plqcd_gauge *gf, void *out, const void *in, void *tmp_o, bool dagger) const {
@@ -111,7 +117,26 @@ struct Op {
         PLQCD_TRY(hop(gf, tmp_o, in, PLQCD_ODD, fin));
         return hop(gf, out, tmp_o, PLQCD_EVEN, fout, in, -kappa * kappa, 1.0);
     }
+    // the same with the sum h in the second hop's epilogue
+    int mhat_sum(const plqcd_gauge *gf, void *out, const void *in, void *tmp_o, bool dagger, const HopSum &h,
+                 const int *halt = nullptr) const {
+        unsigned fin = dagger ? PLQCD_DSLASH_G5_IN : 0u, fout = dagger ? PLQCD_DSLASH_G5_OUT : 0u;
+        PLQCD_TRY(hop(gf, tmp_o, in, PLQCD_ODD, fin, nullptr, 1.0, 0.0, halt));
+        return launch_hop_sum(g, s, call(gf, out, tmp_o, PLQCD_EVEN, fout, in, -kappa * kappa, 1.0, halt), h, red);
+    }
 };
+
+HopSum sum_of(HopSumKind kind, RedOp op, const void *c = nullptr, void *rvec = nullptr, int out_prec = PLQCD_F64,
+              CgReport *report = nullptr) {
+    HopSum h;
+    h.report = report;
+    h.kind = kind;
+    h.op = op;
+    h.c = c;
+    h.rvec = rvec;
+    h.out_prec = out_prec;
+    return h;
+}
 
 }  // namespace
 
@@ -150,7 +175,7 @@ extern "C" int plqcd_invert_cg(plqcd_lattice *lat, const plqcd_gauge *g64, const
     const size_t bs = spinor_parity_bytes(g.Vh, ps);
     const size_t bx = spinor_parity_bytes(g.Vh, xprec);
     auto al = [](size_t n) { return (n + 255) & ~(size_t)255; };
-    const size_t need = 5 * al(b64) + 5 * al(bs) + al(bx) + al(red_scratch_bytes());
+    const size_t need = 3 * al(b64) + 5 * al(bs) + al(bx) + al(red_scratch_bytes(g.Vh));
     void *ws = nullptr;
     PLQCD_TRY(lattice_workspace(lat, need, &ws));
     char *w = static_cast<char *>(ws);
@@ -159,23 +184,29 @@ extern "C" int plqcd_invert_cg(plqcd_lattice *lat, const plqcd_gauge *g64, const
         w += al(n);
         return p;
     };
-    void *bprime = take(b64), *rhs = take(b64), *r64 = take(b64), *t64 = take(b64), *tmp64 = take(b64);
+    void *bprime = take(b64), *t64 = take(b64), *tmp64 = take(b64);
     void *rs = take(bs), *p = take(bs), *Ap = take(bs), *t = take(bs), *tmps = take(bs);
     void *xs = take(bx);
-    void *redmem = take(red_scratch_bytes());
-    PLQCD_CUDA_TRY(cudaMemsetAsync(redmem, 0, red_scratch_bytes(), s));
-    RedScratch red = red_scratch_from(redmem);
+    void *redmem = take(red_scratch_bytes(g.Vh));
+    PLQCD_CUDA_TRY(cudaMemsetAsync(redmem, 0, red_scratch_bytes(g.Vh), s));
+    RedScratch red = red_scratch_from(redmem, g.Vh);
+    // page-locked: the state as last read, its start values, and one report
+    // per iteration in flight
     void *hblock = nullptr;
     PLQCD_TRY(lattice_host_block(lat, &hblock));
+    static_assert(2 * sizeof(CgState) + 2 * sizeof(CgReport) <= kHostBlockBytes, "solver states");
     CgState *hst = static_cast<CgState *>(hblock);
+    CgReport *report = reinterpret_cast<CgReport *>(hst + 2);
     auto read_state = [&]() -> int {
         PLQCD_CUDA_TRY(cudaMemcpyAsync(hst, red.state, sizeof(CgState), cudaMemcpyDeviceToHost, s));
         PLQCD_CUDA_TRY(cudaStreamSynchronize(s));
         return PLQCD_OK;
     };
 
-    Op op{g, s, prm->kappa};
+    Op op{g, s, prm->kappa, red};
     cudaEvent_t e0 = lat->ev0, e1 = lat->ev1;
+    for (cudaEvent_t &ev : lat->iter_event)
+        if (!ev) PLQCD_CUDA_TRY(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
     cudaEventRecord(e0, s);
     int rc = PLQCD_OK;
     plqcd_cg_info inf;
@@ -185,112 +216,110 @@ extern "C" int plqcd_invert_cg(plqcd_lattice *lat, const plqcd_gauge *g64, const
 
     do {
         const bool mixed = ps != PLQCD_F64;
-        // b' = b_e + kappa H_eo b_o ; rhs = Mhat^dag b'
-        if ((rc = op.hop(g64, bprime, b_odd, PLQCD_EVEN, 0, b_even, prm->kappa, 1.0))) break;
-        if ((rc = blas_norm2(g, s, bprime, PLQCD_F64, red, RED_AUX))) break;
-        if (!mixed && (rc = op.mhat(g64, rhs, bprime, tmp64, true))) break;
-        if ((rc = read_state())) break;
-        bp2 = hst->aux;
-        if (!(bp2 > 0)) {  // zero source: zero solution
-            cudaMemsetAsync(x_even, 0, b64, s);
-            rc = op.hop(g64, x_odd, x_even, PLQCD_ODD, 0, b_odd, prm->kappa, 1.0);
-            inf.converged = 1;
+        CgState *init = hst + 1;
+        memset(init, 0, sizeof *init);
+        init->target = prm->tol * prm->tol;  // RED_RR_INIT makes it tol^2 |rhs|^2
+        init->delta2 = prm->delta * prm->delta;
+        init->mixed = mixed;
+        // a sloppy recursion that stops reducing its residual (16-bit storage
+        // with a tiny delta) would never trigger an update: force one after
+        // this many iterations without
+        init->max_run = 100;
+        if (cudaMemcpyAsync(red.state, init, sizeof *init, cudaMemcpyHostToDevice, s) != cudaSuccess) {
+            rc = set_error(PLQCD_ERR_CUDA, "plqcd_invert_cg: state upload failed");
             break;
         }
-        // x = 0, r = p = rhs. The sloppy solution x_s is not cleared: while
-        // `fresh` it counts as zero, and its next update writes it unread
-        cudaMemsetAsync(x_even, 0, b64, s);
-        bool fresh = true;
+        // b' = b_e + kappa H_eo b_o ; r = p = rhs = Mhat^dag b'
+        if ((rc = launch_hop_sum(g, s, Op::call(g64, bprime, b_odd, PLQCD_EVEN, 0, b_even, prm->kappa, 1.0, nullptr),
+                                 sum_of(HOP_NORM, RED_AUX), red)))
+            break;
+        const HopSum rhs_sum = sum_of(HOP_NORM, RED_RR_INIT);
         if (mixed) {
             // the sloppy recursion starts from rhs in sloppy precision, so
             // the sloppy operator computes it; convergence is decided on the
             // FP64 Schur residual of b', which does not use rhs
             if ((rc = launch_spinor_convert(g, s, t, ps, bprime, PLQCD_F64))) break;
-            if ((rc = op.mhat(gs, rs, t, tmps, true))) break;
-            if ((rc = blas_norm2(g, s, rs, ps, red, RED_RR_INIT))) break;
-            if (cudaMemcpyAsync(p, rs, bs, cudaMemcpyDeviceToDevice, s) != cudaSuccess) {
-                rc = set_error(PLQCD_ERR_CUDA, "plqcd_invert_cg: device copy failed");
+            if ((rc = op.mhat_sum(gs, rs, t, tmps, true, rhs_sum))) break;
+            inf.sloppy_hops += 2;
+        } else if ((rc = op.mhat_sum(g64, rs, bprime, tmp64, true, rhs_sum))) {
+            break;
+        }
+        if (cudaMemcpyAsync(p, rs, bs, cudaMemcpyDeviceToDevice, s) != cudaSuccess) {
+            rc = set_error(PLQCD_ERR_CUDA, "plqcd_invert_cg: device copy failed");
+            break;
+        }
+        cudaMemsetAsync(x_even, 0, b64, s);
+        if ((rc = read_state())) break;
+        bp2 = hst->aux;
+        if (!(bp2 > 0)) {  // zero source: zero solution
+            rc = op.hop(g64, x_odd, x_even, PLQCD_ODD, 0, b_odd, prm->kappa, 1.0);
+            inf.sloppy_hops = 0;
+            inf.converged = 1;
+            break;
+        }
+
+        // One iteration, all of it queued at once: Ap = Mhat^dag Mhat p with
+        // |t|^2 = |Mhat p|^2 and r -= alpha Ap, |r|^2 in the hops' epilogues,
+        // then x_s += alpha p, p = r + beta p. The |r|^2 sum decides whether
+        // a reliable update is due; then the p step, and every kernel of the
+        // iteration queued after, does nothing. So the host queues iteration
+        // it + 1 before it reads what iteration `it` came to, and the device
+        // does not wait for it. The outcome reaches the host as a store of the
+        // summing kernel to page-locked memory: a copy between the kernels
+        // held up the stream for 5 us.
+        // The sloppy solution x_s is not cleared: while `fresh` it counts as
+        // zero, and its next update writes it unread.
+        const int *halt = &red.state->halt;
+        auto queue = [&](int it, bool fresh) -> int {
+            PLQCD_TRY(op.mhat_sum(gs, t, p, tmps, false, sum_of(HOP_NORM, RED_ALPHA), halt));
+            PLQCD_TRY(op.mhat_sum(gs, Ap, t, tmps, true,
+                                  sum_of(HOP_UPDATE, RED_RR, nullptr, rs, ps, &report[it & 1]), halt));
+            PLQCD_CUDA_TRY(cudaEventRecord(lat->iter_event[it & 1], s));
+            return blas_cg_p_x(g, s, p, rs, ps, xs, xprec, fresh ? 1 : 2, red);
+        };
+        bool fresh = true;  // before the iteration whose outcome is read next
+        if ((rc = queue(1, fresh))) break;
+        for (int it = 1; it <= prm->max_iter; it++) {
+            if (it < prm->max_iter && (rc = queue(it + 1, false))) break;
+            const cudaError_t e = cudaEventSynchronize(lat->iter_event[it & 1]);
+            if (e != cudaSuccess) {
+                rc = set_error(PLQCD_ERR_CUDA, "plqcd_invert_cg: %s", cudaGetErrorString(e));
                 break;
             }
-            inf.sloppy_hops += 2;
-        } else {
-            if ((rc = blas_norm2(g, s, rhs, PLQCD_F64, red, RED_RR_INIT))) break;
-            if ((rc = launch_spinor_convert(g, s, rs, ps, rhs, PLQCD_F64))) break;
-            if ((rc = launch_spinor_convert(g, s, p, ps, rhs, PLQCD_F64))) break;
-        }
-        if ((rc = read_state())) break;
-        const double rhs2 = hst->rr;
-        double maxrr = hst->rr;
-        double target = prm->tol * prm->tol * rhs2;  // normal-equation trigger for convergence checks
-        const double delta2 = prm->delta * prm->delta;
-        // a sloppy recursion that stops reducing its residual (16-bit storage
-        // with a tiny delta) would never trigger an update: force one after
-        // this many iterations without
-        const int max_sloppy_run = 100;
-        int last_reliable = 0;
-
-        for (int it = 1; it <= prm->max_iter; it++) {
-            // Ap = Mhat^dag Mhat p ; pAp = |Mhat p|^2
-            if ((rc = op.mhat(gs, t, p, tmps, false))) break;
-            if ((rc = blas_norm2(g, s, t, ps, red, RED_ALPHA))) break;
-            if ((rc = op.mhat(gs, Ap, t, tmps, true))) break;
-            // r -= alpha Ap ; |r|^2. The solution update x_s += alpha p of
-            // this iteration runs in the p update below (which reads p
-            // anyway), or in the fold of a reliable update
-            if ((rc = blas_cg_update_r(g, s, rs, Ap, ps, red))) break;
+            const CgReport now = report[it & 1];
             inf.sloppy_hops += 4;
             inf.iterations = it;
-            if ((rc = read_state())) break;
-            const double rr = hst->rr;
-            if (!std::isfinite(rr)) {
+            if (!std::isfinite(now.rr)) {
                 rc = set_error(PLQCD_ERR_NOCONV, "plqcd_invert_cg: residual is not finite at iteration %d", it);
                 break;
             }
-            const bool reliable = (mixed && rr < delta2 * maxrr) || rr <= target || it - last_reliable >= max_sloppy_run;
-            if (reliable) {
-                // defect correction: x += x_s + alpha p, then the Schur
-                // residual b' - Mhat x in FP64 (for the mixed solve written
-                // only in the sloppy format: the restart needs nothing more)
-                if ((rc = blas_accum(g, s, x_even, xs, xprec, fresh, p, ps, red))) break;
-                fresh = true;
-                if ((rc = op.mhat(g64, t64, x_even, tmp64, false))) break;
-                if (mixed)
-                    rc = blas_sub_norm2_to(g, s, t, ps, bprime, t64, red, RED_SR2);
-                else
-                    rc = blas_sub_norm2(g, s, r64, bprime, t64, red, RED_SR2);
-                if (rc) break;
-                inf.f64_hops += 2;
-                inf.reliable_updates++;
-                last_reliable = it;
-                if ((rc = read_state())) break;
-                sr2 = hst->sr2;
-                if (prm->verbose)
-                    fprintf(stderr, "plqcd cg: it %d reliable update, |r_schur|/|b'| = %.3e\n", it, sqrt(sr2 / bp2));
-                if (sr2 <= prm->tol * prm->tol * bp2) {
-                    inf.converged = 1;
-                    break;
-                }
-                // restart the recursion from r = Mhat^dag (b' - Mhat x). The
-                // FP64 residual above decides convergence; the restart
-                // direction only needs the sloppy operator's accuracy
-                if (mixed) {
-                    if ((rc = op.mhat(gs, rs, t, tmps, true))) break;
-                    if ((rc = blas_norm2(g, s, rs, ps, red, RED_RR_TRUE))) break;
-                    inf.sloppy_hops += 2;
-                } else {
-                    if ((rc = op.mhat(g64, t64, r64, tmp64, true))) break;
-                    if ((rc = blas_norm2(g, s, t64, PLQCD_F64, red, RED_RR_TRUE))) break;
-                    if ((rc = launch_spinor_convert(g, s, rs, ps, t64, PLQCD_F64))) break;
-                    inf.f64_hops += 2;
-                }
-                if ((rc = read_state())) break;
-                maxrr = hst->rr;
-                if (hst->rr <= target) target *= 0.25;
-            } else {
-                maxrr = std::max(maxrr, rr);
+            if (!now.halt) {
+                fresh = false;
+                continue;
             }
-            if ((rc = blas_cg_p_x(g, s, p, rs, ps, xs, xprec, reliable ? 0 : (fresh ? 1 : 2), red))) break;
-            if (!reliable) fresh = false;
+            // reliable update, defect correction: x += x_s + alpha p, then
+            // the Schur residual b' - Mhat x in FP64, stored in the sloppy
+            // format (the restart needs nothing more)
+            if ((rc = blas_accum(g, s, x_even, xs, xprec, fresh, p, ps, red))) break;
+            fresh = true;
+            if ((rc = op.mhat_sum(g64, t, x_even, tmp64, false, sum_of(HOP_RESID, RED_SR2, bprime, nullptr, ps)))) break;
+            inf.f64_hops += 2;
+            inf.reliable_updates++;
+            if ((rc = read_state())) break;
+            sr2 = hst->sr2;
+            if (prm->verbose)
+                fprintf(stderr, "plqcd cg: it %d reliable update, |r_schur|/|b'| = %.3e\n", it, sqrt(sr2 / bp2));
+            if (sr2 <= prm->tol * prm->tol * bp2) {
+                inf.converged = 1;
+                break;
+            }
+            // restart the recursion from r = Mhat^dag (b' - Mhat x). The FP64
+            // residual above decides convergence; the restart direction only
+            // needs the sloppy operator's accuracy
+            if ((rc = op.mhat_sum(mixed ? gs : g64, rs, t, tmps, true, sum_of(HOP_NORM, RED_RR_TRUE)))) break;
+            (mixed ? inf.sloppy_hops : inf.f64_hops) += 2;
+            if ((rc = blas_cg_p_x(g, s, p, rs, ps, xs, xprec, 0, red))) break;
+            if (it < prm->max_iter && (rc = queue(it + 1, fresh))) break;
         }
         if (rc) break;
         if (!inf.converged) {
@@ -303,27 +332,21 @@ extern "C" int plqcd_invert_cg(plqcd_lattice *lat, const plqcd_gauge *g64, const
         cudaEventRecord(e1, s);
         end_recorded = true;
         // full-lattice residual |b - D x| / |b|, D x = x - kappa H x
-        double r2 = 0, b2 = 0;
-        if ((rc = op.hop(g64, t64, x_odd, PLQCD_EVEN, 0, x_even, -prm->kappa, 1.0))) break;
-        if ((rc = blas_sub_norm2(g, s, r64, b_even, t64, red, RED_AUX))) break;
+        if ((rc = launch_hop_sum(g, s, Op::call(g64, t64, x_odd, PLQCD_EVEN, 0, x_even, -prm->kappa, 1.0, nullptr),
+                                 sum_of(HOP_CHECK, RED_CHECK_E, b_even), red)))
+            break;
+        if ((rc = launch_hop_sum(g, s, Op::call(g64, t64, x_even, PLQCD_ODD, 0, x_odd, -prm->kappa, 1.0, nullptr),
+                                 sum_of(HOP_CHECK, RED_CHECK_O, b_odd), red)))
+            break;
         if ((rc = read_state())) break;
-        r2 += hst->aux;
-        if ((rc = op.hop(g64, t64, x_even, PLQCD_ODD, 0, x_odd, -prm->kappa, 1.0))) break;
-        if ((rc = blas_sub_norm2(g, s, r64, b_odd, t64, red, RED_AUX))) break;
-        if ((rc = read_state())) break;
-        r2 += hst->aux;
-        if ((rc = blas_norm2(g, s, b_even, PLQCD_F64, red, RED_AUX))) break;
-        if ((rc = read_state())) break;
-        b2 += hst->aux;
-        if ((rc = blas_norm2(g, s, b_odd, PLQCD_F64, red, RED_AUX))) break;
-        if ((rc = read_state())) break;
-        b2 += hst->aux;
-        inf.true_residual = sqrt(r2 / b2);
+        inf.true_residual = sqrt((hst->check[0] + hst->check[2]) / (hst->check[1] + hst->check[3]));
         inf.schur_residual = sqrt(sr2 / bp2);
     } while (0);
 
     if (!end_recorded) cudaEventRecord(e1, s);
-    cudaEventSynchronize(e1);
+    // nothing queued is left behind: an iteration queued ahead still reads x
+    // and writes the page-locked reports
+    cudaStreamSynchronize(s);
     float ms = 0;
     cudaEventElapsedTime(&ms, e0, e1);
     inf.seconds = ms / 1e3;

@@ -33,6 +33,7 @@ namespace plqcd {
 
 int launch_dslash_ahead(cudaStream_t s, const dev::DslashArgs &a, int prec, int recon, bool xpay, bool full,
                         bool joined, bool deep);
+int build_args(const Geom &g, const DslashCall &c, dev::DslashArgs &a);
 
 namespace dev {
 
@@ -96,6 +97,7 @@ __global__ void __launch_bounds__(256) k_dslash_pipe(const DslashArgs a) {
     extern __shared__ uint4 smem[];
     constexpr int NS = SIO::NSLOT + LIO::NSLOT;
     const int B = blockDim.x;
+    if (a.halt && *a.halt) return;
     int par;
     long h;
     if (FULL) {
@@ -230,7 +232,6 @@ static int env_int(const char *name, int dflt) {
 static int dispatch(const Geom &g, cudaStream_t s, const DslashCall &c, const dev::DslashArgs &a, int variant,
                     int block);
 
-static int build_args(const Geom &g, const DslashCall &c, dev::DslashArgs &a);
 static int tune_dslash(const Geom &g, cudaStream_t s, const DslashCall &c, const dev::DslashArgs &a,
                        const char *key);
 
@@ -274,7 +275,7 @@ int launch_dslash(const Geom &g, cudaStream_t s, const DslashCall &c) {
     return rc;
 }
 
-static int build_args(const Geom &g, const DslashCall &c, dev::DslashArgs &a) {
+int build_args(const Geom &g, const DslashCall &c, dev::DslashArgs &a) {
     PLQCD_TRY(check_field_ptr(c.out, "dslash"));
     PLQCD_TRY(check_field_ptr(c.in, "dslash"));
     if (c.full) {
@@ -296,6 +297,7 @@ static int build_args(const Geom &g, const DslashCall &c, dev::DslashArgs &a) {
         a.out[0] = c.out;
     }
     a.x = c.x;
+    a.halt = c.halt;
     a.Vh = g.Vh;
     a.h_begin = c.h_begin;
     a.h_end = c.h_count < 0 ? g.Vh : c.h_begin + c.h_count;
@@ -385,6 +387,7 @@ static int tune_dslash(const Geom &g, cudaStream_t s, const DslashCall &c, const
                 }
             t.out[0] = scratch[0];
             if (c.full) t.out[1] = scratch[1];
+            t.halt = nullptr;
             PLQCD_TRY(dispatch(g, s, c, t, r.variant, r.block));
             PLQCD_CUDA_TRY(cudaStreamSynchronize(s));
             if (dslash_tma_status(true)) return set_error(PLQCD_ERR_CUDA, "dslash: TMA stage wait timed out");
@@ -398,6 +401,7 @@ static int tune_dslash(const Geom &g, cudaStream_t s, const DslashCall &c, const
         dev::DslashArgs t = a;
         t.out[0] = scratch[0];
         if (c.full) t.out[1] = scratch[1];
+        t.halt = nullptr;
         return dispatch(g, s, c, t, r.variant, r.block);
     };
     int rc = tune_launch(key, s, cands, run);

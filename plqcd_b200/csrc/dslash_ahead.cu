@@ -29,7 +29,9 @@
 //                         484 -> 430   the power cap lowers the clock
 #include <cuda_runtime.h>
 
+#include "blas.cuh"
 #include "dslash_core.cuh"
+#include "hop_sum.cuh"
 #include "internal.h"
 #include "raw_loads.cuh"
 
@@ -55,6 +57,91 @@ __device__ __forceinline__ Coords tiled_coords(int s, int par, int L0h, int L1, 
     return c;
 }
 
+// Grids of at most this many blocks finish their sums in the last block to
+// arrive, sparing a launch (2.5 us); above, its 64 threads would take longer
+// over the partials than a kernel of one block of 1024 threads (4 us for the
+// 16384 partials of 32^3x64).
+constexpr long kSumInKernel = 512;
+
+// block sums of (v, w) into the partials [block], [gridDim + block]; every
+// thread of the block takes part
+__device__ __forceinline__ void hop_sum_block(const SumArgs &q, double v, double w, bool two) {
+    __shared__ double ws[2][2];
+    __shared__ bool last;
+    auto warp_sum = [](double t) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        return t;
+    };
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    auto block_sum = [&](double t, double u) {
+        t = warp_sum(t);
+        if (two) u = warp_sum(u);
+        __syncthreads();
+        if (lane == 0) {
+            ws[0][wp] = t;
+            ws[1][wp] = u;
+        }
+        __syncthreads();
+    };
+    block_sum(v, w);
+    CgState st;  // (no other block changes the state before every block has arrived)
+    if (threadIdx.x == 0) {
+        if (q.in_kernel) st = *q.red.state;
+        q.red.partials[blockIdx.x] = ws[0][0] + ws[0][1];
+        if (two) q.red.partials[gridDim.x + blockIdx.x] = ws[1][0] + ws[1][1];
+        last = false;
+        if (q.in_kernel) {
+            __threadfence();
+            last = atomicAdd(q.red.counter, 1u) == gridDim.x - 1;
+        }
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    double t = 0, u = 0;
+    for (int k = threadIdx.x; k < (int)gridDim.x; k += blockDim.x) {
+        t += __ldcg(q.red.partials + k);
+        if (two) u += __ldcg(q.red.partials + gridDim.x + k);
+    }
+    block_sum(t, u);
+    if (threadIdx.x == 0) {
+        red_apply(q.op, ws[0][0] + ws[0][1], ws[1][0] + ws[1][1], st, q.red.state, q.report);
+        *q.red.counter = 0;  // ready for the next sum on this scratch
+    }
+}
+
+// the n partials (of one or two sums) in a fixed order, then the state update
+__global__ void __launch_bounds__(1024) k_hop_sum_finish(RedScratch red, CgReport *report, int n, int two, RedOp op,
+                                                         const int *halt) {
+    __shared__ double ws[2][32];
+    if (halt && *halt) return;
+    CgState st;
+    if (threadIdx.x == 0) st = *red.state;
+    double t = 0, u = 0;
+#pragma unroll 8
+    for (int k = threadIdx.x; k < n; k += 1024) t += red.partials[k];
+    if (two)
+        for (int k = threadIdx.x; k < n; k += 1024) u += red.partials[n + k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        t += __shfl_xor_sync(0xffffffffu, t, o);
+        u += __shfl_xor_sync(0xffffffffu, u, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        ws[0][threadIdx.x >> 5] = t;
+        ws[1][threadIdx.x >> 5] = u;
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    t = u = 0;
+    for (int i = 0; i < 32; i++) {
+        t += ws[0][i];
+        u += ws[1][i];
+    }
+    red_apply(op, t, u, st, red.state, report);
+}
+
 // MODE 0: one parity; 1: with the xpay epilogue; 2: full lattice, the two
 // parities of the same sites in neighbouring blocks; 3: full lattice, the
 // two parities of 32 sites in one block (one warp each), sites in the 2x2x2
@@ -64,9 +151,13 @@ __device__ __forceinline__ Coords tiled_coords(int s, int par, int L0h, int L1, 
 // against 451 with the parities joined in the plain order and 462 in mode 2;
 // 4x2x2 430, 2x4x4 447, 4x4x4 453, 2x8x8 452, half of z x all of t 445;
 // short run 441 against 452 in mode 2).
-template <class SIO, class LIO, int MODE, int DEPTH, int MINB>
-__global__ void __launch_bounds__(kAheadBlock, MINB) k_dslash_ahead(const DslashArgs a) {
+// SUM (mode 1, whole fields): a HopSumKind; OP: the format of its output.
+// Threads past the last site compute on it and add nothing.
+template <class SIO, class LIO, int MODE, int DEPTH, int MINB, int SUM = 0, int OP = PLQCD_F64>
+__global__ void __launch_bounds__(kAheadBlock, MINB) k_dslash_ahead(const DslashArgs a, const SumArgs q) {
     using R = typename SIO::real;
+    static_assert(SUM == 0 || MODE == 1, "sums belong to the xpay epilogue");
+    if (a.halt && *a.halt) return;
     constexpr bool XPAY = MODE == 1, FULL = MODE >= 2;
     int par;
     long h;
@@ -80,7 +171,11 @@ __global__ void __launch_bounds__(kAheadBlock, MINB) k_dslash_ahead(const Dslash
         par = a.out_parity;
         h = a.h_begin + (long)(blockIdx.x / a.nrhs) * kAheadBlock + threadIdx.x;
     }
-    if (h >= a.h_end) return;
+    const bool valid = h < a.h_end;
+    if (!valid) {
+        if (SUM == 0) return;
+        h = a.h_end - 1;
+    }
     const int opp = par ^ 1;
     // selects, not a dynamic index into the parameter arrays (which would
     // copy them to local memory)
@@ -150,7 +245,13 @@ __global__ void __launch_bounds__(kAheadBlock, MINB) k_dslash_ahead(const Dslash
             acc[k] = {ak * acc[k].re, ak * acc[k].im};
         }
     }
-    SIO::store(out, Vh, h, acc);
+    if constexpr (SUM == 0) {
+        SIO::store(out, Vh, h, acc);
+    } else {
+        double v = 0, w = 0;
+        if (valid) sum_epilogue<SIO, SUM, OP>(q, out, Vh, h, acc, v, w);
+        hop_sum_block(q, v, w, SUM == HOP_CHECK);
+    }
 }
 
 template <class SIO, class LIO, int MODE, int DEPTH, int MINB>
@@ -158,7 +259,7 @@ static int launch_ahead_t(cudaStream_t s, const DslashArgs &a) {
     const long per = MODE == 3 ? 32 : kAheadBlock;
     const long nblk = (a.h_end - a.h_begin + per - 1) / per * (MODE == 2 ? 2 : a.nrhs);
     if (nblk > 0x7fffffffL) return set_error(PLQCD_ERR_ARG, "dslash: grid too large");
-    k_dslash_ahead<SIO, LIO, MODE, DEPTH, MINB><<<(unsigned)nblk, kAheadBlock, 0, s>>>(a);
+    k_dslash_ahead<SIO, LIO, MODE, DEPTH, MINB><<<(unsigned)nblk, kAheadBlock, 0, s>>>(a, SumArgs{});
     PLQCD_CUDA_TRY(cudaGetLastError());
     return PLQCD_OK;
 }
@@ -173,6 +274,29 @@ static int launch_ahead_m(cudaStream_t s, const DslashArgs &a, bool deep) {
         if (deep) return launch_ahead_t<S, L, MODE, 2, 8>(s, a);
         return launch_ahead_t<S, L, MODE, 1, P == PLQCD_F32 ? 8 : 10>(s, a);
     }
+}
+
+template <int P, int RC>
+static int launch_sum_pr(cudaStream_t s, const DslashArgs &a, const SumArgs &q, unsigned nblk, const HopSum &h) {
+    using S = SpinorIO<P>;
+    using L = LinkIO<P, RC>;
+    constexpr int D = P == PLQCD_F32 ? 2 : 1, B = P == PLQCD_F64 ? 4 : P == PLQCD_F32 ? 8 : 10;
+    void (*k)(const DslashArgs, const SumArgs) = nullptr;
+    if (h.kind == HOP_NORM) k = k_dslash_ahead<S, L, 1, D, B, HOP_NORM>;
+    if (h.kind == HOP_UPDATE) k = k_dslash_ahead<S, L, 1, D, B, HOP_UPDATE>;
+    if constexpr (P == PLQCD_F64) {
+        if (h.kind == HOP_CHECK) k = k_dslash_ahead<S, L, 1, D, B, HOP_CHECK>;
+        if (h.kind == HOP_RESID) switch (h.out_prec) {
+                case PLQCD_F64: k = k_dslash_ahead<S, L, 1, D, B, HOP_RESID, PLQCD_F64>; break;
+                case PLQCD_F32: k = k_dslash_ahead<S, L, 1, D, B, HOP_RESID, PLQCD_F32>; break;
+                case PLQCD_F16: k = k_dslash_ahead<S, L, 1, D, B, HOP_RESID, PLQCD_F16>; break;
+                case PLQCD_BF16: k = k_dslash_ahead<S, L, 1, D, B, HOP_RESID, PLQCD_BF16>; break;
+            }
+    }
+    if (!k) return set_error(PLQCD_ERR_ARG, "hop with a sum: kind %d not available for precision %d", (int)h.kind, P);
+    k<<<nblk, kAheadBlock, 0, s>>>(a, q);
+    PLQCD_CUDA_TRY(cudaGetLastError());
+    return PLQCD_OK;
 }
 
 template <int P, int RC>
@@ -202,6 +326,37 @@ int launch_dslash_ahead(cudaStream_t s, const dev::DslashArgs &a, int prec, int 
         default:
             return set_error(PLQCD_ERR_ARG, "dslash: unsupported precision/reconstruction %d/%d", prec, recon);
     }
+}
+
+size_t hop_sum_partials(long Vh) { return 2 * (size_t)((Vh + dev::kAheadBlock - 1) / dev::kAheadBlock); }
+
+int build_args(const Geom &g, const DslashCall &c, dev::DslashArgs &a);
+
+int launch_hop_sum(const Geom &g, cudaStream_t s, const DslashCall &c, const HopSum &h, const RedScratch &r) {
+    dev::DslashArgs a{};
+    PLQCD_TRY(build_args(g, c, a));
+    if (!c.x || c.full || c.nrhs != 1 || a.h_begin != 0 || a.h_end != g.Vh || (c.flags & PLQCD_DSLASH_COMPAT))
+        return set_error(PLQCD_ERR_ARG, "hop with a sum: whole one-parity fields with an xpay operand only");
+    if ((h.kind == HOP_UPDATE && !h.rvec) || ((h.kind == HOP_RESID || h.kind == HOP_CHECK) && !h.c))
+        return set_error(PLQCD_ERR_ARG, "hop with a sum: operand missing");
+    const long nblk = (g.Vh + dev::kAheadBlock - 1) / dev::kAheadBlock;
+    const dev::SumArgs q{h.c, h.rvec, r, h.report, h.op, nblk <= dev::kSumInKernel};
+    int rc;
+    switch (c.prec * 100 + c.recon) {
+        case PLQCD_F64 * 100 + 18: rc = dev::launch_sum_pr<PLQCD_F64, 18>(s, a, q, (unsigned)nblk, h); break;
+        case PLQCD_F64 * 100 + 12: rc = dev::launch_sum_pr<PLQCD_F64, 12>(s, a, q, (unsigned)nblk, h); break;
+        case PLQCD_F32 * 100 + 18: rc = dev::launch_sum_pr<PLQCD_F32, 18>(s, a, q, (unsigned)nblk, h); break;
+        case PLQCD_F32 * 100 + 12: rc = dev::launch_sum_pr<PLQCD_F32, 12>(s, a, q, (unsigned)nblk, h); break;
+        case PLQCD_F16 * 100 + 12: rc = dev::launch_sum_pr<PLQCD_F16, 12>(s, a, q, (unsigned)nblk, h); break;
+        case PLQCD_BF16 * 100 + 12: rc = dev::launch_sum_pr<PLQCD_BF16, 12>(s, a, q, (unsigned)nblk, h); break;
+        default:
+            return set_error(PLQCD_ERR_ARG, "dslash: unsupported precision/reconstruction %d/%d", c.prec, c.recon);
+    }
+    if (rc == PLQCD_OK && !q.in_kernel) {
+        dev::k_hop_sum_finish<<<1, 1024, 0, s>>>(r, h.report, (int)nblk, h.kind == HOP_CHECK, h.op, c.halt);
+        PLQCD_CUDA_TRY(cudaGetLastError());
+    }
+    return rc;
 }
 
 }  // namespace plqcd

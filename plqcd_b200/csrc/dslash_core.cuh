@@ -29,6 +29,7 @@ struct DslashArgs {
     // only: blocks cover the RHS of a site range consecutively (RHS fastest)
     int nrhs;
     long fbytes;
+    const int *halt;  // nothing to do once *halt is set (null: no such flag)
 };
 
 // Two FP32 lanes in one register pair, each operation one packed sm_100

@@ -81,6 +81,7 @@ struct plqcd_lattice {
     void *host_block = nullptr;
     cudaStream_t solve_stream = nullptr;
     cudaEvent_t solve_event = nullptr;
+    cudaEvent_t iter_event[2] = {nullptr, nullptr};  // iterations in flight of the single-RHS solver
 };
 
 struct plqcd_gauge {
@@ -137,6 +138,9 @@ struct DslashCall {
     long h_begin = 0, h_count = -1;
     // single parity: in/out/x are blocks of nrhs fields back to back
     int nrhs = 1;
+    // device flag: a launch that finds it set does nothing (null: none). The
+    // TMA kernels do not look; their output is then written all the same
+    const int *halt = nullptr;
 };
 int launch_dslash(const Geom &g, cudaStream_t s, const DslashCall &c);
 // TMA-staged hop (dslash_tma.cu): variant 1000 * kind + 100 * nstage + ny
