@@ -9,6 +9,8 @@
 
 #include "blas.cuh"
 #include "device_fields.cuh"
+#include "pdl.cuh"
+#include "raw_loads.cuh"
 
 namespace plqcd {
 
@@ -50,20 +52,21 @@ template <int P, int XP, int XMODE>
 __global__ void __launch_bounds__(kBlasBlock) k_cg_p_x(void *p, const void *rs, void *xs, long Vh, const CgState *st) {
     using R = typename SpinorIO<P>::real;
     using RX = typename SpinorIO<XP>::real;
+    pdl_start();
     if (XMODE && st->halt) return;
     const R beta = (R)st->beta;
     const RX ax = (RX)st->alpha;
     for (long h = (long)blockIdx.x * blockDim.x + threadIdx.x; h < Vh; h += (long)gridDim.x * blockDim.x) {
         cx<R> pv[12], rv[12];
-        SpinorIO<P>::load(p, Vh, h, pv);
-        SpinorIO<P>::load(rs, Vh, h, rv);
+        load_coherent<SpinorIO<P>>(p, Vh, h, pv);
+        load_coherent<SpinorIO<P>>(rs, Vh, h, rv);
         if (XMODE) {
             cx<RX> xv[12];
             if (XMODE == 1) {
 #pragma unroll
                 for (int k = 0; k < 12; k++) xv[k] = {RX(0), RX(0)};
             } else {
-                SpinorIO<XP>::load(xs, Vh, h, xv);
+                load_coherent<SpinorIO<XP>>(xs, Vh, h, xv);
             }
 #pragma unroll
             for (int k = 0; k < 12; k++)
@@ -125,9 +128,9 @@ int blas_cg_p_x(const Geom &g, cudaStream_t s, void *p, const void *rs, int prec
         return set_error(PLQCD_ERR_ARG, "blas_cg_p_x: solution accumulator must be F64 or F32");
 #define G(P, XP)                                                                                        \
     switch (xmode) {                                                                                    \
-        case 0: dev::k_cg_p_x<P, XP, 0><<<nb, kBlasBlock, 0, s>>>(p, rs, xs, g.Vh, r.state); break;     \
-        case 1: dev::k_cg_p_x<P, XP, 1><<<nb, kBlasBlock, 0, s>>>(p, rs, xs, g.Vh, r.state); break;     \
-        default: dev::k_cg_p_x<P, XP, 2><<<nb, kBlasBlock, 0, s>>>(p, rs, xs, g.Vh, r.state); break;   \
+        case 0: return launch_overlapped(dev::k_cg_p_x<P, XP, 0>, (unsigned)nb, kBlasBlock, s, p, rs, xs, g.Vh, r.state);     \
+        case 1: return launch_overlapped(dev::k_cg_p_x<P, XP, 1>, (unsigned)nb, kBlasBlock, s, p, rs, xs, g.Vh, r.state);     \
+        default: return launch_overlapped(dev::k_cg_p_x<P, XP, 2>, (unsigned)nb, kBlasBlock, s, p, rs, xs, g.Vh, r.state);   \
     }
 #define F(P)                         \
     if (xprec == PLQCD_F64) {        \

@@ -33,6 +33,7 @@
 #include "dslash_core.cuh"
 #include "hop_sum.cuh"
 #include "internal.h"
+#include "pdl.cuh"
 #include "raw_loads.cuh"
 
 namespace plqcd {
@@ -115,6 +116,7 @@ __device__ __forceinline__ void hop_sum_block(const SumArgs &q, double v, double
 __global__ void __launch_bounds__(1024) k_hop_sum_finish(RedScratch red, CgReport *report, int n, int two, RedOp op,
                                                          const int *halt) {
     __shared__ double ws[2][32];
+    pdl_start();
     if (halt && *halt) return;
     CgState st;
     if (threadIdx.x == 0) st = *red.state;
@@ -173,7 +175,10 @@ __global__ void __launch_bounds__(kAheadBlock, MINB) k_dslash_ahead(const Dslash
     }
     const bool valid = h < a.h_end;
     if (!valid) {
-        if (SUM == 0) return;
+        if (SUM == 0) {
+            pdl_start();
+            return;
+        }
         h = a.h_end - 1;
     }
     const int opp = par ^ 1;
@@ -194,6 +199,8 @@ __global__ void __launch_bounds__(kAheadBlock, MINB) k_dslash_ahead(const Dslash
     }
     int nb[8];
     neighbour_sites(c, xh, a.L0, a.L0h, a.L1, a.L2, a.L3, nb);
+    pdl_start();
+    if (a.halt && *a.halt) return;
 
     constexpr int S = DEPTH + 1;
     RawSpinor<SIO> rs[S];
@@ -259,9 +266,7 @@ static int launch_ahead_t(cudaStream_t s, const DslashArgs &a) {
     const long per = MODE == 3 ? 32 : kAheadBlock;
     const long nblk = (a.h_end - a.h_begin + per - 1) / per * (MODE == 2 ? 2 : a.nrhs);
     if (nblk > 0x7fffffffL) return set_error(PLQCD_ERR_ARG, "dslash: grid too large");
-    k_dslash_ahead<SIO, LIO, MODE, DEPTH, MINB><<<(unsigned)nblk, kAheadBlock, 0, s>>>(a, SumArgs{});
-    PLQCD_CUDA_TRY(cudaGetLastError());
-    return PLQCD_OK;
+    return launch_overlapped(k_dslash_ahead<SIO, LIO, MODE, DEPTH, MINB>, (unsigned)nblk, kAheadBlock, s, a, SumArgs{});
 }
 
 template <int P, int RC, int MODE>
@@ -294,9 +299,7 @@ static int launch_sum_pr(cudaStream_t s, const DslashArgs &a, const SumArgs &q, 
             }
     }
     if (!k) return set_error(PLQCD_ERR_ARG, "hop with a sum: kind %d not available for precision %d", (int)h.kind, P);
-    k<<<nblk, kAheadBlock, 0, s>>>(a, q);
-    PLQCD_CUDA_TRY(cudaGetLastError());
-    return PLQCD_OK;
+    return launch_overlapped(k, nblk, kAheadBlock, s, a, q);
 }
 
 template <int P, int RC>
@@ -352,10 +355,8 @@ int launch_hop_sum(const Geom &g, cudaStream_t s, const DslashCall &c, const Hop
         default:
             return set_error(PLQCD_ERR_ARG, "dslash: unsupported precision/reconstruction %d/%d", c.prec, c.recon);
     }
-    if (rc == PLQCD_OK && !q.in_kernel) {
-        dev::k_hop_sum_finish<<<1, 1024, 0, s>>>(r, h.report, (int)nblk, h.kind == HOP_CHECK, h.op, c.halt);
-        PLQCD_CUDA_TRY(cudaGetLastError());
-    }
+    if (rc == PLQCD_OK && !q.in_kernel)
+        rc = launch_overlapped(dev::k_hop_sum_finish, 1, 1024, s, r, h.report, (int)nblk, h.kind == HOP_CHECK, h.op, c.halt);
     return rc;
 }
 

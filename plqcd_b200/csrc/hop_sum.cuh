@@ -3,6 +3,7 @@
 
 #include "blas.cuh"
 #include "device_fields.cuh"
+#include "raw_loads.cuh"
 
 namespace plqcd {
 namespace dev {
@@ -38,14 +39,14 @@ __device__ __forceinline__ void sum_epilogue(const SumArgs &q, void *out, long V
     } else if constexpr (SUM == HOP_UPDATE) {
         const R al = (R)q.red.state->alpha;
         cx<R> rv[12];
-        SIO::load(q.rvec, Vh, h, rv);
+        load_coherent<SIO>(q.rvec, Vh, h, rv);
 #pragma unroll
         for (int k = 0; k < 12; k++) rv[k] = {fma(-al, acc[k].re, rv[k].re), fma(-al, acc[k].im, rv[k].im)};
         SIO::store(q.rvec, Vh, h, rv);
         v = site_norm2(rv);
     } else {
         cx<R> cv[12];
-        SIO::load(q.c, Vh, h, cv);
+        load_coherent<SIO>(q.c, Vh, h, cv);
         if (SUM == HOP_CHECK) w = site_norm2(cv);
 #pragma unroll
         for (int k = 0; k < 12; k++) cv[k] = csub(cv[k], acc[k]);

@@ -5,7 +5,9 @@
 // the current one keeps the stored form in registers meanwhile: a 16-bit
 // spinor takes 13 registers, its converted form 24. The loads are volatile
 // asm statements, so they stay in the order written (ahead of the
-// arithmetic) instead of being moved down to their uses.
+// arithmetic) instead of being moved down to their uses, and ordinary ones
+// (not the non-coherent path), so a kernel may read what the one it overlaps
+// with has written (pdl.cuh).
 #pragma once
 
 #include "device_fields.cuh"
@@ -15,22 +17,22 @@ namespace dev {
 
 __device__ __forceinline__ uint4 ld_v4(const void *p) {
     uint4 v;
-    asm volatile("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
     return v;
 }
 __device__ __forceinline__ uint2 ld_v2(const void *p) {
     uint2 v;
-    asm volatile("ld.global.nc.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+    asm volatile("ld.global.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
     return v;
 }
 __device__ __forceinline__ double2 ld_d2(const void *p) {
     double2 v;
-    asm volatile("ld.global.nc.v2.f64 {%0,%1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+    asm volatile("ld.global.v2.f64 {%0,%1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
     return v;
 }
 __device__ __forceinline__ float ld_f(const void *p) {
     float v;
-    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
     return v;
 }
 
@@ -153,6 +155,18 @@ struct RawLink<LinkIO<PLQCD_F32, 18>> {
         for (int e = 0; e < 9; e++) U[e] = {__uint_as_float(v[e].x), __uint_as_float(v[e].y)};
     }
 };
+
+// a spinor by ordinary loads, its norm applied
+template <class SIO, typename R>
+__device__ __forceinline__ void load_coherent(const void *base, long Vh, long h, cx<R> s[12]) {
+    RawSpinor<SIO> raw;
+    R n;
+    raw.load(base, Vh, (int)h);
+    raw.get(s, n);
+    if (SIO::kScaled)
+#pragma unroll
+        for (int k = 0; k < 12; k++) s[k] = {s[k].re * n, s[k].im * n};
+}
 
 }  // namespace dev
 }  // namespace plqcd

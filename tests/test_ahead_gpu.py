@@ -77,3 +77,31 @@ def test_ahead_f64_against_oracle(cuda, monkeypatch, restatement, dims, config):
     want = restatement.hop("oe", dims, q, u, want)
     got = field_to_host(lat, oe, P.F64, 0) + field_to_host(lat, oo, P.F64, 1)
     assert relmax(got, want) < 1e-14
+
+
+@pytest.mark.parametrize("prec,recon", [(P.F64, 18), (P.F32, 12), (P.F16, 12)])
+@pytest.mark.parametrize("dims", [(2, 2, 2, 2), (4, 6, 8, 10), (16, 16, 16, 32)])
+def test_dependent_launches_back_to_back(cuda, monkeypatch, dims, prec, recon):
+    """Launches that overlap their predecessor's end read all of its output
+    and overwrite none of its input: a chain that hands two buffers back and
+    forth gives the bits of the chain that waits after every launch."""
+    lat = new_lattice(dims)
+    g = P.Gauge(lat, prec, recon)
+    g.random(3)
+    nb = lat.spinor_bytes(prec)
+    start = dev_bytes(nb)
+    lat.spinor_gaussian(start, prec, 0, 8)
+    _force(monkeypatch, 0, 64)
+    got = []
+    for wait in (True, False, False):
+        a, b = start.clone(), dev_bytes(nb)
+        for k in range(40):
+            lat.dslash(g, b, a, 1, prec)
+            if wait:
+                lat.synchronize()
+            lat.dslash_xpay(g, a, b, 0, prec, -0.01, a, 1.0)  # x is overwritten in place
+            if wait:
+                lat.synchronize()
+        lat.synchronize()
+        got.append(a)
+    assert bool((got[0] == got[1]).all()) and bool((got[0] == got[2]).all())
