@@ -5,11 +5,12 @@
 //   direction it loads the link once and applies it to the NR neighbour
 //   spinors (direct loads, or a cp.async ring);
 // - RHS pairs (FP32, F16, BF16): two RHS on the two lanes of packed FP32
-//   instructions, the link loaded, rebuilt and broadcast once per pair;
-//   their xpay form can carry the CG's dot products in its epilogue
-//   (RhsSink, for the batched solver);
+//   instructions, the link loaded, rebuilt and broadcast once per pair, with
+//   loads at the use or a direction ahead in registers; their xpay form can
+//   carry the CG's dot products in its epilogue (RhsSink, for the batched
+//   solver);
 // - FP64 link sharing: a block of RHS warps over 32 sites reads each link
-//   from shared memory;
+//   from shared memory (dslash_mrhs_links.cu);
 // - the single-RHS kernels with the RHS index folded into the grid
 //   (dslash.cu), and the tensor-core kernel (dslash_mrhs_tc.cu).
 // Consecutive blocks cover the RHS tiles of the same sites (tile index
@@ -30,24 +31,16 @@
 
 #include "dslash_core.cuh"
 #include "internal.h"
+#include "mrhs_core.cuh"
+#include "raw_loads.cuh"
 #include "tune.h"
 
 namespace plqcd {
-namespace dev {
 
-struct MrhsArgs {
-    const void *gauge;
-    const char *in;
-    char *out;
-    const char *x;
-    size_t fbytes;
-    int nrhs, ntiles;
-    long Vh;
-    int L0, L0h, L1, L2, L3;
-    int out_parity;
-    double a_up, a_low, b, g5_in;
-    RhsSink sink;  // fused CG sums (RHS-pair kernels, epi > 0)
-};
+// FP64, links of a block in shared memory (dslash_mrhs_links.cu)
+int launch_mrhs_links(const Geom &g, cudaStream_t s, int recon, const dev::MrhsArgs &a, int warps, bool xpay);
+
+namespace dev {
 
 template <class SIO, class LIO, int NR, bool XPAY>
 __global__ void __launch_bounds__(256) k_dslash_mrhs(const MrhsArgs a) {
@@ -209,13 +202,6 @@ __global__ void __launch_bounds__(256) k_dslash_mrhs_pipe(const MrhsArgs a) {
     }
 }
 
-__device__ __forceinline__ double sq_sum(const cx<float> v[12]) {
-    double s = 0;
-#pragma unroll
-    for (int k = 0; k < 12; k++) s += (double)v[k].re * v[k].re + (double)v[k].im * v[k].im;
-    return s;
-}
-
 // the block's per-RHS sums v0 (RHS r0) and v1 (r0 + 1) into the partials
 // [RHS][site block]; k_sink_finish adds them up
 __device__ void sink_block(const MrhsArgs &a, int r0, bool two, double v0, double v1) {
@@ -273,56 +259,6 @@ __global__ void __launch_bounds__(1024) k_sink_finish(const RhsSink k, int nsb) 
     }
 }
 
-// epilogue of the RHS-pair kernels: scale (and xpay with x from xload(j,
-// xv)), then EPI 0 / 1: store (1: |out|^2 to the sink); EPI 2: r -= alpha
-// out in place, |r|^2 to the sink (out is not stored). Threads past the last
-// site (valid false) only take part in the sums.
-template <class SIO, bool XPAY, int EPI, class XLoad>
-__device__ __forceinline__ void pair_epilogue(const MrhsArgs &a, int r0, bool two, int h, bool valid,
-                                              const cx<f2> acc[12], XLoad xload) {
-    const float aup = (float)a.a_up, alow = (float)a.a_low, b = (float)a.b;
-    double v[2] = {0.0, 0.0};
-#pragma unroll
-    for (int j = 0; j < 2; j++) {
-        if ((j == 1 && !two) || !valid) break;
-        cx<float> o[12];
-#pragma unroll
-        for (int k = 0; k < 12; k++) o[k] = lane(acc[k], j);
-        if (XPAY) {
-            cx<float> xv[12];
-            xload(j, xv);
-#pragma unroll
-            for (int k = 0; k < 12; k++) {
-                const float ak = k < 6 ? aup : alow;
-                o[k] = {fmaf(ak, o[k].re, b * xv[k].re), fmaf(ak, o[k].im, b * xv[k].im)};
-            }
-        } else {
-#pragma unroll
-            for (int k = 0; k < 12; k++) {
-                const float ak = k < 6 ? aup : alow;
-                o[k] = {ak * o[k].re, ak * o[k].im};
-            }
-        }
-        if (EPI == 2) {
-            const int f = r0 + j;
-            if (a.sink.active[f]) {
-                const float al = (float)a.sink.alpha[f];
-                char *rf = a.sink.rvec + (size_t)f * a.fbytes;
-                cx<float> rv[12];
-                SIO::load(rf, a.Vh, h, rv);
-#pragma unroll
-                for (int k = 0; k < 12; k++) rv[k] = {fmaf(-al, o[k].re, rv[k].re), fmaf(-al, o[k].im, rv[k].im)};
-                SIO::store(rf, a.Vh, h, rv);
-                v[j] = sq_sum(rv);
-            }
-        } else {
-            SIO::store(a.out + (size_t)(r0 + j) * a.fbytes, a.Vh, h, o);
-            if (EPI == 1 || EPI == 3) v[j] = sq_sum(o);
-        }
-    }
-    if (EPI > 0 && EPI < 4) sink_block(a, r0, two, v[0], v[1]);
-}
-
 // RHS-pair kernel: one thread, one output site, two right-hand sides on the
 // two lanes of Blackwell's packed FP32 instructions (FFMA2 / FMUL2 / FADD2):
 // lane 0 carries RHS r0, lane 1 RHS r0 + 1. The link is loaded, converted,
@@ -331,8 +267,8 @@ __device__ __forceinline__ void pair_epilogue(const MrhsArgs &a, int r0, bool tw
 // compute_dir with the same rounding, so the results are the bits of the
 // other kernels. An odd last RHS runs in both lanes and is stored once.
 // (FP32-computing formats: F32, F16, BF16.)
-template <class SIO, class LIO, bool XPAY, int MINB = 1, int EPI = 0>
-__global__ void __launch_bounds__(256, MINB) k_dslash_mrhs_pair(const MrhsArgs a) {
+template <class SIO, class LIO, bool XPAY, int EPI = 0>
+__global__ void __launch_bounds__(256, 2) k_dslash_mrhs_pair(const MrhsArgs a) {
     static_assert(std::is_same<typename SIO::real, float>::value, "packed lanes hold FP32");
     const int tile = blockIdx.x % a.ntiles;
     const int hh = (blockIdx.x / a.ntiles) * blockDim.x + threadIdx.x;
@@ -377,247 +313,124 @@ __global__ void __launch_bounds__(256, MINB) k_dslash_mrhs_pair(const MrhsArgs a
         for (int e = 0; e < 12; e++) s[e] = zip(sa[e], sb[e]);
         compute_dir_n<false, SIO::kScaled, f2>(d, acc, s, Ub, sg, f2(na, nbv));
     }
+    double v[2];
     pair_epilogue<SIO, XPAY, EPI>(a, r0, two, h, valid, acc, [&](int j, cx<float> xv[12]) {
         SIO::load(a.x + (size_t)(r0 + j) * a.fbytes, Vh, h, xv);
-    });
+    }, v);
+    if (EPI > 0 && EPI < 4) sink_block(a, r0, two, v[0], v[1]);
 }
 
-// Pipelined RHS-pair kernel: the link and the two neighbour spinors of a
-// direction are copied global->shared with cp.async into slots private to
-// the thread, ST directions ahead of the one being computed (as in
-// k_dslash_mrhs_pipe), so the loads stay in flight without holding the
-// registers the packed arithmetic needs.
-template <class SIO, class LIO, int ST, bool XPAY, int MINB = 1, int EPI = 0>
-__global__ void __launch_bounds__(256, MINB) k_dslash_mrhs_pair_pipe(const MrhsArgs a) {
+// RHS-pair kernel with the next direction's link and two neighbour spinors
+// (at the end the two xpay operands) already on their way into registers, in
+// their stored form. 168 registers, 12 warps per SM; the heavy FMA pipe, which
+// also converts the 16-bit values, is the nearest bound. 24^3x48, 8 RHS: F16 156
+// us, where the form above takes 166 and a cp.async ring (taken out) took 170;
+// F32-18 206 both; BF16 xpay 188 against 182: the tuner decides. Links
+// converted once per block and kept in shared memory as operand pairs took
+// 170: the blocks' start-up is exposed.
+constexpr int kPairAheadBlock = 64;
+template <class SIO, class LIO, bool XPAY, int EPI = 0>
+__global__ void __launch_bounds__(kPairAheadBlock, 6) k_dslash_mrhs_pair_ahead(const MrhsArgs a) {
     static_assert(std::is_same<typename SIO::real, float>::value, "packed lanes hold FP32");
-    extern __shared__ uint4 smem[];
-    constexpr int NS = LIO::NSLOT + 2 * SIO::NSLOT;
-    const int B = blockDim.x;
     const int tile = blockIdx.x % a.ntiles;
-    const int hh = (blockIdx.x / a.ntiles) * B + threadIdx.x;
+    const int hh = (blockIdx.x / a.ntiles) * kPairAheadBlock + threadIdx.x;
     const bool valid = hh < a.Vh;
-    // no block-level barrier below except the sums of EPI 1-3, in which
-    // every thread (a past-the-end one on the last site) takes part
-    if ((EPI == 0 || EPI == 4) && !valid) return;
+    if ((EPI == 0 || EPI == 4) && !valid) return;  // (EPI 1-3: every thread takes part in the sums)
     const int h = valid ? hh : (int)a.Vh - 1;
-    // restart hops (EPI 3, 4): a pair of retired RHS has nothing to compute (whole block)
-    if (EPI >= 3 && !a.sink.active[2 * tile] && !(2 * tile + 1 < a.nrhs && a.sink.active[2 * tile + 1])) return;
     const int r0 = 2 * tile;
+    // restart hops (EPI 3, 4): a pair of retired RHS has nothing to compute (whole block)
+    if (EPI >= 3 && !a.sink.active[r0] && !(r0 + 1 < a.nrhs && a.sink.active[r0 + 1])) return;
     const bool two = r0 + 1 < a.nrhs;
     const char *in0 = a.in + (size_t)r0 * a.fbytes;
     const char *in1 = two ? in0 + a.fbytes : in0;
+    const char *x0 = XPAY ? a.x + (size_t)r0 * a.fbytes : nullptr;
+    const char *x1 = two ? x0 + a.fbytes : x0;
     const int par = a.out_parity, opp = par ^ 1;
     const long Vh = a.Vh;
-    const int L0h = a.L0h, L1 = a.L1, L2 = a.L2, L3 = a.L3;
-    const Coords c = site_coords(h, par, L0h, L1, L2);
-    const int xh = h - c.row * L0h;
+    const Coords c = site_coords(h, par, a.L0h, a.L1, a.L2);
+    const int xh = h - c.row * a.L0h;
     int nb[8];
-    neighbour_sites(c, xh, a.L0, L0h, L1, L2, L3, nb);
+    neighbour_sites(c, xh, a.L0, a.L0h, a.L1, a.L2, a.L3, nb);
     const f2 sg((float)a.g5_in);
-
-    const int stride = B * 16;
-    const uint32_t s_thread = smem_addr(smem) + threadIdx.x * 16;
-    // k-th direction of dir_at into slot k % ST: link, then RHS r0, r0 + 1
+    RawSpinor<SIO> ra[2], rb[2];
+    RawLink<LIO> rl[2];
     auto issue = [&](int k) {
-        const int d = dir_at(k);
-        const uint32_t s0 = s_thread + (uint32_t)((k % ST) * NS) * stride;
-        if (d < 4)
-            LIO::issue(a.gauge, Vh, par, d, h, s0, stride);
-        else
-            LIO::issue(a.gauge, Vh, opp, d - 4, nb[d], s0, stride);
-        SIO::issue(in0, Vh, nb[d], s0 + (uint32_t)LIO::NSLOT * stride, stride);
-        SIO::issue(in1, Vh, nb[d], s0 + (uint32_t)(LIO::NSLOT + SIO::NSLOT) * stride, stride);
-    };
-    // xpay: the two x spinors of the output site go in with the first
-    // direction, into slots after the ring, so the epilogue does not wait
-    const uint32_t s_x = s_thread + (uint32_t)(ST * NS) * stride;
-#pragma unroll
-    for (int k = 0; k < ST; k++) {
-        issue(k);
-        if (XPAY && k == 0) {
-            SIO::issue(a.x + (size_t)r0 * a.fbytes, Vh, h, s_x, stride);
-            SIO::issue(a.x + (size_t)(two ? r0 + 1 : r0) * a.fbytes, Vh, h, s_x + SIO::NSLOT * stride, stride);
+        if (k < 8) {
+            const int d = dir_at(k);
+            if (d < 4)
+                rl[k & 1].load(a.gauge, Vh, par, d, h);
+            else
+                rl[k & 1].load(a.gauge, Vh, opp, d - 4, nb[d]);
+            ra[k & 1].load(in0, Vh, nb[d]);
+            rb[k & 1].load(in1, Vh, nb[d]);
+        } else if (XPAY) {
+            ra[0].load(x0, Vh, h);
+            rb[0].load(x1, Vh, h);
         }
-        cp_async_commit();
-    }
+    };
     cx<f2> acc[12];
 #pragma unroll
     for (int k = 0; k < 12; k++) acc[k] = {f2(0.f), f2(0.f)};
+    issue(0);
 #pragma unroll
     for (int k = 0; k < 8; k++) {
-        const int d = dir_at(k);
-        cp_async_wait<ST - 1>();
-        const uint4 *s0 = smem + threadIdx.x + (k % ST) * NS * B;
+        issue(k + 1);
         cx<float> U[9];
-        LIO::load_staged(s0, B, U);
+        rl[k & 1].get(U);
         cx<f2> Ub[9];
 #pragma unroll
         for (int e = 0; e < 9; e++) Ub[e] = {f2(U[e].re), f2(U[e].im)};
         cx<float> sa[12], sb[12];
         float na, nbv;
-        SIO::load_staged_raw(s0 + LIO::NSLOT * B, B, sa, na);
-        SIO::load_staged_raw(s0 + (LIO::NSLOT + SIO::NSLOT) * B, B, sb, nbv);
+        ra[k & 1].get(sa, na);
+        rb[k & 1].get(sb, nbv);
         cx<f2> s[12];
 #pragma unroll
         for (int e = 0; e < 12; e++) s[e] = zip(sa[e], sb[e]);
-        compute_dir_n<false, SIO::kScaled, f2>(d, acc, s, Ub, sg, f2(na, nbv));
-        // the slot just consumed is refilled only after its values were used
-        if (k + ST < 8) issue(k + ST);
-        cp_async_commit();
+        compute_dir_n<false, SIO::kScaled, f2>(dir_at(k), acc, s, Ub, sg, f2(na, nbv));
     }
+    double v[2];
     pair_epilogue<SIO, XPAY, EPI>(a, r0, two, h, valid, acc, [&](int j, cx<float> xv[12]) {
-        SIO::load_staged(smem + threadIdx.x + (ST * NS + j * SIO::NSLOT) * B, B, xv);
-    });
+        float n;
+        (j ? rb[0] : ra[0]).get(xv, n);
+        if (SIO::kScaled)
+#pragma unroll
+            for (int k = 0; k < 12; k++) xv[k] = {xv[k].re * n, xv[k].im * n};
+    }, v);
+    if (EPI > 0 && EPI < 4) sink_block(a, r0, two, v[0], v[1]);
 }
 
-// ST = 0: direct loads (k_dslash_mrhs_pair), else the cp.async pipeline of
-// depth ST; MINB = 2 caps the registers at 128 a thread (more warps per SM)
+// ahead: k_dslash_mrhs_pair_ahead (its own block size), else direct loads at
+// the use with at most 128 registers a thread.
 // epi > 0 (fused CG sums, xpay hops only): see RhsSink
-template <class SIO, class LIO, int ST, int MINB = 1>
-static int launch_pair(const Geom &g, cudaStream_t s, MrhsArgs a, int block, bool xpay, int epi = 0) {
+template <class SIO, class LIO>
+static int launch_pair(const Geom &g, cudaStream_t s, MrhsArgs a, bool ahead, int block, bool xpay, int epi) {
     if constexpr (!std::is_same<typename SIO::real, float>::value) {
         return set_error(PLQCD_ERR_ARG, "dslash_mrhs: the RHS-pair kernel computes in FP32 only");
     } else {
         if (g.Vh >= (1L << 31)) return set_error(PLQCD_ERR_ARG, "dslash_mrhs: lattice too large for 32-bit sites");
+        if (ahead) block = kPairAheadBlock;
         if (epi && ((epi == 4) == xpay || block > 256 || block % 32))
             return set_error(PLQCD_ERR_ARG, "dslash_mrhs: fused epilogue %d does not fit this hop", epi);
         a.ntiles = (a.nrhs + 1) / 2;
         const long nblk = (g.Vh + block - 1) / block * a.ntiles;
         if (nblk > 0x7fffffffL) return set_error(PLQCD_ERR_ARG, "dslash_mrhs: grid too large");
-        if constexpr (ST == 0) {
-            auto k = epi == 4 ? k_dslash_mrhs_pair<SIO, LIO, false, MINB, 4>
-                   : epi == 3 ? k_dslash_mrhs_pair<SIO, LIO, true, MINB, 3>
-                   : epi == 2 ? k_dslash_mrhs_pair<SIO, LIO, true, MINB, 2>
-                   : epi == 1 ? k_dslash_mrhs_pair<SIO, LIO, true, MINB, 1>
-                   : xpay     ? k_dslash_mrhs_pair<SIO, LIO, true, MINB, 0>
-                              : k_dslash_mrhs_pair<SIO, LIO, false, MINB, 0>;
-            k<<<(unsigned)nblk, block, 0, s>>>(a);
-        } else {
-            constexpr int NS = LIO::NSLOT + 2 * SIO::NSLOT;
-            const size_t smem = (size_t)(ST * NS + (xpay ? 2 * SIO::NSLOT : 0)) * 16 * block;
-            if (smem > 227 * 1024) return set_error(PLQCD_ERR_ARG, "dslash_mrhs: %zu bytes of shared memory", smem);
-            auto k = epi == 4 ? k_dslash_mrhs_pair_pipe<SIO, LIO, ST, false, MINB, 4>
-                   : epi == 3 ? k_dslash_mrhs_pair_pipe<SIO, LIO, ST, true, MINB, 3>
-                   : epi == 2 ? k_dslash_mrhs_pair_pipe<SIO, LIO, ST, true, MINB, 2>
-                   : epi == 1 ? k_dslash_mrhs_pair_pipe<SIO, LIO, ST, true, MINB, 1>
-                   : xpay     ? k_dslash_mrhs_pair_pipe<SIO, LIO, ST, true, MINB, 0>
-                              : k_dslash_mrhs_pair_pipe<SIO, LIO, ST, false, MINB, 0>;
-            // (the fused sums hold static shared memory, so opt in to what this launch needs)
-            PLQCD_TRY(smem_optin((const void *)k, smem));
-            k<<<(unsigned)nblk, block, smem, s>>>(a);
-        }
+        auto k = ahead ? (epi == 4 ? k_dslash_mrhs_pair_ahead<SIO, LIO, false, 4>
+                        : epi == 3 ? k_dslash_mrhs_pair_ahead<SIO, LIO, true, 3>
+                        : epi == 2 ? k_dslash_mrhs_pair_ahead<SIO, LIO, true, 2>
+                        : epi == 1 ? k_dslash_mrhs_pair_ahead<SIO, LIO, true, 1>
+                        : xpay     ? k_dslash_mrhs_pair_ahead<SIO, LIO, true, 0>
+                                   : k_dslash_mrhs_pair_ahead<SIO, LIO, false, 0>)
+                       : (epi == 4 ? k_dslash_mrhs_pair<SIO, LIO, false, 4>
+                        : epi == 3 ? k_dslash_mrhs_pair<SIO, LIO, true, 3>
+                        : epi == 2 ? k_dslash_mrhs_pair<SIO, LIO, true, 2>
+                        : epi == 1 ? k_dslash_mrhs_pair<SIO, LIO, true, 1>
+                        : xpay     ? k_dslash_mrhs_pair<SIO, LIO, true, 0>
+                                   : k_dslash_mrhs_pair<SIO, LIO, false, 0>);
+        k<<<(unsigned)nblk, block, 0, s>>>(a);
         PLQCD_CUDA_TRY(cudaGetLastError());
         return PLQCD_OK;
     }
-}
-
-// FP64 link-sharing kernel: a block of NRB warps covers 32 consecutive
-// output sites for NRB right-hand sides (warp w = RHS w of the block's
-// group, lane = site). Per direction the block copies the links of its 32
-// sites into shared memory once (cp.async, each warp a share of the
-// planes) and every warp copies its own neighbour spinors; all NRB warps
-// then read the links from shared memory. A link crosses L2->SM once per
-// NRB RHS instead of once per RHS, which is what bounds the FP64 multi-RHS
-// hop when each RHS is a separate block. The ring holds ST directions with
-// one block barrier per direction: stage k + ST - 1 is refilled into the
-// slot of stage k - 1 after the barrier that every warp passes once it has
-// computed k - 1. Threads past the last site or RHS copy in-bounds data and
-// store nothing. Same arithmetic, so the same bits, as the other kernels.
-template <class LIO, int NRB, int ST, bool XPAY>
-__global__ void __launch_bounds__(32 * NRB) k_dslash_mrhs_f64blk(const MrhsArgs a) {
-    using SIO = SpinorIO<PLQCD_F64>;
-    constexpr int NT = 32 * NRB;
-    constexpr int LP = LIO::NE;            // link planes, 16 bytes a site each
-    constexpr int LB = LP * 32;            // link slots of the block's sites
-    constexpr int STAGE = LB + SIO::NSLOT * NT;
-    extern __shared__ uint4 smem[];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int grp = blockIdx.x % a.ntiles;
-    const int h0 = (blockIdx.x / a.ntiles) * 32;
-    const int r = grp * NRB + w;
-    const bool rhs_ok = r < a.nrhs;
-    const int h = h0 + lane;
-    const bool site_ok = h < a.Vh;
-    const int hc = site_ok ? h : h0;  // h0 < Vh: out-of-range lanes copy a valid site
-    const char *in = a.in + (size_t)(rhs_ok ? r : 0) * a.fbytes;
-    const int par = a.out_parity, opp = par ^ 1;
-    const long Vh = a.Vh;
-    const int L0h = a.L0h, L1 = a.L1, L2 = a.L2, L3 = a.L3;
-    const Coords c = site_coords(hc, par, L0h, L1, L2);
-    const int xh = hc - c.row * L0h;
-    int nb[8];
-    neighbour_sites(c, xh, a.L0, L0h, L1, L2, L3, nb);
-    const double sg = a.g5_in;
-
-    const uint32_t base = smem_addr(smem);
-    // direction k of dir_at into ring slot k % ST: link planes e = w, w + NRB,
-    // ... of site lane (the link of the lane's own site, or of its backward
-    // neighbour), then this thread's neighbour spinor
-    auto issue = [&](int k) {
-        const int d = dir_at(k);
-        const uint32_t st = base + (uint32_t)((k % ST) * STAGE) * 16u;
-        const int lsite = d < 4 ? hc : nb[d];
-        const int lpar = d < 4 ? par : opp;
-        const double2 *lp = static_cast<const double2 *>(a.gauge) + ((long)(lpar * 4 + (d & 3)) * LP) * Vh + lsite;
-#pragma unroll
-        for (int e = w; e < LP; e += NRB) cp_async16_cg(st + (uint32_t)(e * 32 + lane) * 16u, lp + e * Vh);
-        SIO::issue(in, Vh, nb[d], st + (uint32_t)(LB + threadIdx.x) * 16u, NT * 16);
-    };
-#pragma unroll
-    for (int k = 0; k < ST - 1; k++) {
-        issue(k);
-        cp_async_commit();
-    }
-    cx<double> acc[12];
-#pragma unroll
-    for (int k = 0; k < 12; k++) acc[k] = {0.0, 0.0};
-#pragma unroll
-    for (int k = 0; k < 8; k++) {
-        cp_async_wait<ST - 2>();  // this thread's copies of stage k
-        __syncthreads();          // everyone's copies of stage k; everyone done with k - 1
-        if (k + ST - 1 < 8) issue(k + ST - 1);
-        cp_async_commit();
-        const uint4 *stg = smem + (k % ST) * STAGE;
-        cx<double> U[9], s[12];
-        double n;
-        LIO::load_staged(stg + lane, 32, U);
-        SIO::load_staged_raw(stg + LB + threadIdx.x, NT, s, n);
-        compute_dir_n<false, false, double>(dir_at(k), acc, s, U, sg, n);
-    }
-    if (!site_ok || !rhs_ok) return;
-    const double aup = a.a_up, alow = a.a_low;
-    if (XPAY) {
-        cx<double> xv[12];
-        SIO::load(a.x + (size_t)r * a.fbytes, Vh, h, xv);
-        const double b = a.b;
-#pragma unroll
-        for (int k = 0; k < 12; k++) {
-            const double ak = k < 6 ? aup : alow;
-            acc[k] = {fma(ak, acc[k].re, b * xv[k].re), fma(ak, acc[k].im, b * xv[k].im)};
-        }
-    } else {
-#pragma unroll
-        for (int k = 6; k < 12; k++) acc[k] = {alow * acc[k].re, alow * acc[k].im};
-#pragma unroll
-        for (int k = 0; k < 6; k++) acc[k] = {aup * acc[k].re, aup * acc[k].im};
-    }
-    SIO::store(a.out + (size_t)r * a.fbytes, Vh, h, acc);
-}
-
-template <class LIO, int NRB, int ST>
-static int launch_f64blk(const Geom &g, cudaStream_t s, MrhsArgs a, bool xpay) {
-    if (g.Vh >= (1L << 31)) return set_error(PLQCD_ERR_ARG, "dslash_mrhs: lattice too large for 32-bit sites");
-    a.ntiles = (a.nrhs + NRB - 1) / NRB;
-    const long nblk = (g.Vh + 31) / 32 * a.ntiles;
-    if (nblk > 0x7fffffffL) return set_error(PLQCD_ERR_ARG, "dslash_mrhs: grid too large");
-    constexpr int STAGE = LIO::NE * 32 + SpinorIO<PLQCD_F64>::NSLOT * 32 * NRB;
-    const size_t smem = (size_t)ST * STAGE * 16;
-    if (smem > 227 * 1024) return set_error(PLQCD_ERR_ARG, "dslash_mrhs: %zu bytes of shared memory", smem);
-    auto k = xpay ? k_dslash_mrhs_f64blk<LIO, NRB, ST, true> : k_dslash_mrhs_f64blk<LIO, NRB, ST, false>;
-    PLQCD_TRY(smem_optin((const void *)k, 227 * 1024));
-    k<<<(unsigned)nblk, 32 * NRB, smem, s>>>(a);
-    PLQCD_CUDA_TRY(cudaGetLastError());
-    return PLQCD_OK;
 }
 
 template <class SIO, class LIO, int NR, int ST>
@@ -661,28 +474,22 @@ static int launch_pr(const Geom &g, cudaStream_t s, const MrhsArgs &a, int nr, i
         case 1042:
             if constexpr (P != PLQCD_F64) return launch_nr_pipe<S, L, 4, 2>(g, s, a, block, xpay);
             break;
-        // 2002: RHS-pair kernel on packed FP32 lanes; 2022 / 2032: its
-        // cp.async pipeline of depth 2 / 3
-        case 2002: return launch_pair<S, L, 0>(g, s, a, block, xpay, epi);
-        case 2022: return launch_pair<S, L, 2>(g, s, a, block, xpay, epi);
-        case 2032: return launch_pair<S, L, 3>(g, s, a, block, xpay, epi);
-        // 4000 + 100 * ring depth + RHS per block: FP64 link-sharing kernel
-        case 4208:
+        // RHS-pair kernels on packed FP32 lanes: 2200 loads ahead, 2102 at the
+        // use (tuning files may hold 2002 to 2122, forms that these replaced)
+        case 2200:
+        case 2022:
+        case 2032:
+        case 2122: return launch_pair<S, L>(g, s, a, true, block, xpay, epi);
+        case 2102:
+        case 2002: return launch_pair<S, L>(g, s, a, false, block, xpay, epi);
+        // 4200 + RHS per block: FP64, links in shared memory (43xx in older files)
+        case 4202:
         case 4204:
-        case 4308:
+        case 4208:
         case 4304:
-            if constexpr (P == PLQCD_F64) {
-                switch (nr) {
-                    case 4208: return launch_f64blk<L, 8, 2>(g, s, a, xpay);
-                    case 4204: return launch_f64blk<L, 4, 2>(g, s, a, xpay);
-                    case 4308: return launch_f64blk<L, 8, 3>(g, s, a, xpay);
-                    default: return launch_f64blk<L, 4, 3>(g, s, a, xpay);
-                }
-            }
+        case 4308:
+            if constexpr (P == PLQCD_F64) return launch_mrhs_links(g, s, RC, a, nr % 100, xpay);
             break;
-        // 2102 / 2122: the same with at most 128 registers a thread
-        case 2102: return launch_pair<S, L, 0, 2>(g, s, a, block, xpay, epi);
-        case 2122: return launch_pair<S, L, 2, 2>(g, s, a, block, xpay, epi);
         case 1: return launch_nr<S, L, 1>(g, s, a, block, xpay);
         case 2: return launch_nr<S, L, 2>(g, s, a, block, xpay);
         case 4:
@@ -725,7 +532,7 @@ static int launch_mrhs_tma(const Geom &g, cudaStream_t s, const void *gauge, int
 
 // tuner key of a multi-RHS hop
 static void mrhs_key(char *key, size_t n, const Geom &g, int prec, int recon, int nrhs, bool xpay) {
-    snprintf(key, n, "%sdslash_mrhs|p%d|r%d|%s|n%d|%dx%dx%dx%d", device_tag().c_str(), prec, recon,
+    snprintf(key, n, "%sdslash_mrhs|p%d|r%d|%s|n%d|%dx%dx%dx%d|c2", device_tag().c_str(), prec, recon,
              xpay ? "xpay" : "plain", nrhs, g.L[0], g.L[1], g.L[2], g.L[3]);
 }
 
@@ -767,8 +574,9 @@ static int mrhs_args(const Geom &g, const void *gauge, int prec, void *out, cons
     return PLQCD_OK;
 }
 
-// the RHS-pair configuration that runs this xpay hop with fused sums: the
-// environment's, else the tuned one (false when it is another kernel)
+// the RHS-pair configuration that runs this hop with fused sums: the
+// environment's (false when it is another kernel), else the tuned one or the
+// load-ahead form
 static bool mrhs_sink_config(const Geom &g, int prec, int recon, int nrhs, TuneResult *t, bool xpay = true) {
     const char *ev = getenv("PLQCD_MRHS_VARIANT");
     if (ev && *ev) {
@@ -781,7 +589,14 @@ static bool mrhs_sink_config(const Geom &g, int prec, int recon, int nrhs, TuneR
         if (!tune_lookup(key, t)) return false;
     }
     const int v = t->variant;
-    return v == 2002 || v == 2022 || v == 2032 || v == 2102 || v == 2122;
+    if (v == 2002 || v == 2102) return true;
+    // not a pair kernel: one is at most a few percent behind (F32-12, 5 RHS at
+    // 24^3x48: 137 against 131 us), and the passes its sums spare are more
+    const bool forced = ev && *ev;
+    if (v != 2200 && v != 2022 && v != 2032 && v != 2122 && forced) return false;
+    t->variant = 2200;
+    t->block = dev::kPairAheadBlock;
+    return true;
 }
 
 bool dslash_mrhs_sink_ok(const Geom &g, int prec, int recon, int nrhs, int *variant, int *block) {
@@ -867,10 +682,11 @@ int launch_dslash_mrhs(const Geom &g, cudaStream_t s, const void *gauge, int pre
     // size 1, 2, 4), and the single-RHS kernels with the RHS index folded
     // into the grid, RHS fastest, so the blocks of one site range run
     // together and share links through L2 (variant = 100 + single-RHS
-    // variant: 0 direct loads, 2/3 cp.async pipeline depth)
+    // variant: 0 loads ahead in registers, 2/3 cp.async pipeline depth)
     std::vector<TuneResult> cands;
     for (int v : {102, 100, 103})
         for (int blk : {64, 128, 256}) {
+            if (v == 100 && blk == 256) continue;  // (64: depth 1, 128: depth 2)
             TuneResult t;
             t.variant = v;
             t.block = blk;
@@ -897,22 +713,23 @@ int launch_dslash_mrhs(const Geom &g, cudaStream_t s, const void *gauge, int pre
                         t.block = blk;
                         cands.push_back(t);
                     }
-    // FP64: the link-sharing block kernel (4000 + 100 * depth + RHS per block)
-    if (prec == PLQCD_F64 && nrhs >= 4)
-        for (int v : {4208, 4204, 4308, 4304}) {
+    // FP64: links of a block in shared memory (4200 + RHS per block)
+    if (prec == PLQCD_F64 && nrhs >= 2)
+        for (int v : {4202, 4204}) {
             if ((v % 100) > nrhs) continue;
             TuneResult t;
             t.variant = v;
             t.block = 32 * (v % 100);
             cands.push_back(t);
         }
-    for (int nr : {2022, 2122, 2032, 2002, 2102, 1022, 1042, 2, 1, 4}) {
+    for (int nr : {2200, 2102, 1022, 1042, 2, 1, 4}) {
         const bool pair = nr >= 2000;
         if (pair && (prec == PLQCD_F64 || nrhs < 2)) continue;
         const int tile = pair ? 2 : nr >= 1000 ? (nr / 10) % 10 : nr;
         if (tile == 4 && prec == PLQCD_F64) continue;
         if (tile > nrhs && tile != 1) continue;
         for (int blk : {64, 128, 256}) {
+            if (nr == 2200 && blk != 64) continue;
             TuneResult t;
             t.variant = nr;
             t.block = blk;

@@ -1,0 +1,155 @@
+// dslash_mrhs_links.cu -- FP64 multi-RHS hop: the links of a block's sites in
+// shared memory, the spinors ahead in registers (sm_100a).
+//
+// A block of n warps covers 32 output sites for n right-hand sides (warp =
+// RHS, lane = site). The warps share out the eight directions and copy their
+// links into shared memory once (cp.async, each lane its own site's slots);
+// after one barrier every warp computes its RHS, the next direction's
+// neighbour spinor (and at the end the xpay operand) on its way into
+// registers meanwhile. A link crosses L2->SM once per n RHS, which with the
+// spinors is what bounds the hop: at 16^3x32 with 12 RHS and n = 2, 2.1 kB per
+// site and RHS, 12 TB/s. Same arithmetic, so the same bits, as the other
+// kernels. Threads past the last site or RHS copy in-bounds data and store
+// nothing.
+//
+// Two RHS per block are best (232 registers, 8 warps per SM in 4 blocks whose
+// start-ups overlap): us at 16^3x32 with 12 RHS / 24^3x48 with 4 RHS, xpay,
+// 1: 172 / 319, 2: 134 / 240, 4: 136 / 245, 8: 173 / 385, at 200 registers 139
+// and 141 for n = 2 and 4. Before: the TMA kernel with RHS tiles 144, one
+// thread per RHS 264; links in shared memory with the spinors beside them 263 /
+// 650.
+#include <cuda_runtime.h>
+
+#include "dslash_core.cuh"
+#include "internal.h"
+#include "mrhs_core.cuh"
+#include "raw_loads.cuh"
+
+namespace plqcd {
+namespace dev {
+
+constexpr int kLinkSlots = 8 * 9 * 32;  // 16-byte slots: [direction of dir_at][element][site]
+
+// the links of the directions in `mine` at the block's 32 sites, copied by
+// the calling warp (its lanes are the sites)
+template <class LIO>
+__device__ __forceinline__ void issue_links(uint4 *lk, unsigned mine, const void *gauge, long Vh, int par, int h,
+                                            const int nb[8]) {
+    const uint32_t s0 = smem_addr(lk) + (threadIdx.x & 31) * 16;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        const int d = dir_at(k);
+        if (mine >> k & 1)
+            LIO::issue(gauge, Vh, d < 4 ? par : par ^ 1, d & 3, d < 4 ? h : nb[d], s0 + k * (9 * 32 * 16), 32 * 16);
+    }
+    cp_async_commit();
+}
+
+// waits for them, rebuilds row 2 of 12-real links in place, and for the block
+template <class LIO>
+__device__ __forceinline__ void finish_links(uint4 *lk, unsigned mine) {
+    const int lane = threadIdx.x & 31;
+    cp_async_wait<0>();
+    if constexpr (LIO::NSLOT < 9)
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            if (!(mine >> k & 1)) continue;
+            uint4 *p = lk + k * (9 * 32) + lane;
+            cx<double> U[9];
+            LIO::load_staged(p, 32, U);
+#pragma unroll
+            for (int e = 6; e < 9; e++) *reinterpret_cast<double2 *>(p + e * 32) = make_double2(U[e].re, U[e].im);
+        }
+    __syncthreads();
+}
+
+template <class LIO, bool XPAY>
+__global__ void __maxnreg__(232) k_mrhs_links_f64(const MrhsArgs a) {
+    using SIO = SpinorIO<PLQCD_F64>;
+    __shared__ uint4 lk[kLinkSlots];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int grp = blockIdx.x % a.ntiles, sb = blockIdx.x / a.ntiles;
+    const int r = grp * nw + w;
+    const bool valid = sb * 32 + lane < a.Vh;
+    const int h = valid ? sb * 32 + lane : (int)a.Vh - 1;
+    const int par = a.out_parity;
+    const long Vh = a.Vh;
+    const Coords c = site_coords(h, par, a.L0h, a.L1, a.L2);
+    const int xh = h - c.row * a.L0h;
+    int nb[8];
+    neighbour_sites(c, xh, a.L0, a.L0h, a.L1, a.L2, a.L3, nb);
+    unsigned mine = 0;
+    for (int k = w; k < 8; k += nw) mine |= 1u << k;
+    issue_links<LIO>(lk, mine, a.gauge, Vh, par, h, nb);
+    const bool has = r < a.nrhs;
+    const char *in = a.in + (size_t)(has ? r : 0) * a.fbytes;
+    const char *x = XPAY ? a.x + (size_t)(has ? r : 0) * a.fbytes : nullptr;
+    RawSpinor<SIO> rs[2];
+    auto issue = [&](int k) {
+        if (k < 8)
+            rs[k & 1].load(in, Vh, nb[dir_at(k)]);
+        else if (XPAY)
+            rs[0].load(x, Vh, h);
+    };
+    issue(0);
+    finish_links<LIO>(lk, mine);
+    if (!has || !valid) return;
+    const double sg = a.g5_in;
+    cx<double> acc[12];
+#pragma unroll
+    for (int k = 0; k < 12; k++) acc[k] = {0.0, 0.0};
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        issue(k + 1);
+        cx<double> U[9], s[12];
+        double n;
+#pragma unroll
+        for (int e = 0; e < 9; e++) {
+            const double2 v = *reinterpret_cast<const double2 *>(lk + (k * 9 + e) * 32 + lane);
+            U[e] = {v.x, v.y};
+        }
+        rs[k & 1].get(s, n);
+        compute_dir_n<false, false, double>(dir_at(k), acc, s, U, sg, n);
+    }
+    const double aup = a.a_up, alow = a.a_low;
+    if (XPAY) {
+        cx<double> xv[12];
+        double n;
+        rs[0].get(xv, n);
+        const double b = a.b;
+#pragma unroll
+        for (int k = 0; k < 12; k++) {
+            const double ak = k < 6 ? aup : alow;
+            acc[k] = {fma(ak, acc[k].re, b * xv[k].re), fma(ak, acc[k].im, b * xv[k].im)};
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < 12; k++) {
+            const double ak = k < 6 ? aup : alow;
+            acc[k] = {ak * acc[k].re, ak * acc[k].im};
+        }
+    }
+    SIO::store(a.out + (size_t)r * a.fbytes, Vh, h, acc);
+}
+
+template <int RC>
+static int launch_links(const Geom &g, cudaStream_t s, MrhsArgs a, int warps, bool xpay) {
+    using L = LinkIO<PLQCD_F64, RC>;
+    a.ntiles = (a.nrhs + warps - 1) / warps;
+    const long nblk = (g.Vh + 31) / 32 * a.ntiles;
+    if (nblk > 0x7fffffffL) return set_error(PLQCD_ERR_ARG, "dslash_mrhs: grid too large");
+    auto k = xpay ? k_mrhs_links_f64<L, true> : k_mrhs_links_f64<L, false>;
+    k<<<(unsigned)nblk, 32 * warps, 0, s>>>(a);
+    PLQCD_CUDA_TRY(cudaGetLastError());
+    return PLQCD_OK;
+}
+
+}  // namespace dev
+
+// FP64 hop of `warps` (1 to 8) RHS per block
+int launch_mrhs_links(const Geom &g, cudaStream_t s, int recon, const dev::MrhsArgs &a, int warps, bool xpay) {
+    if (warps < 1 || warps > 8) return set_error(PLQCD_ERR_ARG, "dslash_mrhs: %d RHS per block", warps);
+    return recon == 18 ? dev::launch_links<18>(g, s, a, warps, xpay) : dev::launch_links<12>(g, s, a, warps, xpay);
+}
+
+}  // namespace plqcd

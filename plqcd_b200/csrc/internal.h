@@ -184,8 +184,8 @@ struct RhsSink {
     const int *active;
     char *rvec;
 };
-// the tuned xpay configuration of this multi-RHS hop is an RHS-pair kernel,
-// so launch_dslash_mrhs_sink can run it
+// launch_dslash_mrhs_sink can run this multi-RHS hop (it is tuned, and not
+// forced to another kernel than an RHS-pair one)
 bool dslash_mrhs_sink_ok(const Geom &g, int prec, int recon, int nrhs, int *variant = nullptr, int *block = nullptr);
 int launch_dslash_mrhs_sink(const Geom &g, cudaStream_t s, const void *gauge, int prec, int recon, void *out,
                             const void *in, int nrhs, int out_parity, unsigned flags, double a, const void *x,

@@ -60,6 +60,35 @@ def test_ahead_same_bits(cuda, monkeypatch, dims, prec, recon):
             assert bool((a == b).all()), (v, k)
 
 
+@pytest.mark.parametrize("nrhs", [1, 2, 3, 5, 9])
+@pytest.mark.parametrize("dims", DIMS)
+@pytest.mark.parametrize("prec,recon", FORMATS)
+def test_multi_rhs_ahead_same_bits(cuda, monkeypatch, dims, prec, recon, nrhs):
+    """The multi-RHS kernels that load ahead (RHS pairs; FP64 with the links
+    of a block in shared memory, 2, 4 and 8 RHS per block, idle warps
+    included) against the single-RHS pipeline kernel."""
+    lat = new_lattice(dims)
+    g = P.Gauge(lat, prec, recon)
+    g.random(17)
+    nb = lat.spinor_bytes(prec)
+    f, x = dev_bytes(nrhs * nb), dev_bytes(nrhs * nb)
+    for r in range(nrhs):
+        lat.spinor_gaussian(f[r * nb:], prec, 1, 50 + r)
+        lat.spinor_gaussian(x[r * nb:], prec, 0, 70 + r)
+    flags = P.DSLASH_G5_IN | P.DSLASH_G5_OUT
+    monkeypatch.setenv("PLQCD_MRHS_BLOCK", "64")
+    got = {}
+    for v in (102, *((4202, 4204, 4208) if prec == P.F64 else (2200, 2102))):
+        monkeypatch.setenv("PLQCD_MRHS_VARIANT", str(v))
+        o = [dev_bytes(nrhs * nb).fill_(7) for _ in range(2)]
+        lat.dslash_mrhs(g, o[0], f, nrhs, 0, prec)
+        lat.dslash_mrhs_xpay(g, o[1], f, nrhs, 0, prec, 0.25, x, -2.0, flags)
+        lat.synchronize()
+        got[v] = o
+    for v, o in got.items():
+        assert bool((o[0] == got[102][0]).all()) and bool((o[1] == got[102][1]).all()), v
+
+
 @pytest.mark.parametrize("dims", DIMS[1:])
 @pytest.mark.parametrize("config", [(0, 64), (21, 64)])
 def test_ahead_f64_against_oracle(cuda, monkeypatch, restatement, dims, config):
