@@ -709,7 +709,7 @@ def run_cg(torch, P, lat, g64, buf, args):
 def run_mrhs(torch, P, lat, g64, args, nrhs=8):
     """Multi-RHS hopping throughput at the benchmark lattice: bytes per site
     and RHS = 2 * spinor + 8 * link / nrhs. For the FP32-computing formats
-    the RHS-pair kernel (variant 2002) and the scalar kernels, and for the
+    the RHS-pair kernels (variants 2200, 2102) and the scalar kernels, and for the
     16-bit ones the tensor-core kernel (3001), are also timed forced (keys
     variant/block), beside the tuner's choice."""
     res = {"nrhs": nrhs}
@@ -749,9 +749,9 @@ def run_mrhs(torch, P, lat, g64, args, nrhs=8):
             res[name]["forced_us"] = forced
         elif prec == P.F64:
             forced = {}
-            # 4xxx: links shared in shared memory; 1xxxxx-8xxxxx: TMA-staged
+            # 42xx: links of a block in shared memory; 1xxxxx-8xxxxx: TMA-staged
             # rows with RHS tiles (100000 * RHS per tile + TMA variant)
-            for v, blk in ((4208, 256), (4204, 128), (4308, 256), (4304, 128), (100, 128), (102, 64), (2, 128),
+            for v, blk in ((4202, 64), (4204, 128), (4208, 256), (100, 64), (102, 64), (2, 128),
                            (1022, 64), (402202, 0), (402102, 0), (404202, 0), (402201, 0), (202202, 0),
                            (802101, 0)):
                 os.environ["PLQCD_MRHS_VARIANT"], os.environ["PLQCD_MRHS_BLOCK"] = str(v), str(blk)
@@ -762,8 +762,7 @@ def run_mrhs(torch, P, lat, g64, args, nrhs=8):
             res[name]["forced_us"] = forced
         else:
             forced = {}
-            cand = [(2002, 64), (2002, 128), (2022, 64), (2022, 128), (2032, 64), (2102, 64), (2102, 128),
-                    (2122, 64), (2122, 128), (102, 128), (2, 128)]
+            cand = [(2200, 64), (2102, 64), (2102, 128), (100, 64), (100, 128), (102, 128), (2, 128)]
             if prec in (P.F16, P.BF16):
                 cand += [(3001, 128), (1042, 128), (1022, 64)]
             for v, blk in cand:

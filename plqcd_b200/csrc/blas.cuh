@@ -144,4 +144,15 @@ int blas_accum(const Geom &g, cudaStream_t s, void *x64, const void *xs, int xpr
 // c.x must be set; with c.halt the launch does nothing once *c.halt is set
 int launch_hop_sum(const Geom &g, cudaStream_t s, const DslashCall &c, const HopSum &h, const RedScratch &r);
 
+// FP64 multi-RHS hop with HOP_RESID or HOP_CHECK per RHS (dslash_mrhs_links.cu):
+// out, in, x and h.c are blocks of nrhs fields (out in the format h.out_prec;
+// not written by HOP_CHECK); sums[nrhs] (HOP_CHECK: sums[2 * nrhs], |z|^2
+// then |c|^2). partials: nrhs * ceil(Vh / 32) doubles, twice that for
+// HOP_CHECK. Meant for nrhs >= 2.
+int launch_mrhs_links_sum(const Geom &g, cudaStream_t s, const plqcd_gauge *gf, void *out, const void *in, int nrhs,
+                          int out_parity, double a, const void *x, double b, const HopSum &h, double *partials,
+                          double *sums);
+
+int preload_mrhs_links_resid(int recon, int out_prec);
+
 }  // namespace plqcd

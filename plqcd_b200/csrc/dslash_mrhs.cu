@@ -32,6 +32,7 @@
 #include "dslash_core.cuh"
 #include "internal.h"
 #include "mrhs_core.cuh"
+#include "pdl.cuh"
 #include "raw_loads.cuh"
 #include "tune.h"
 
@@ -335,11 +336,8 @@ __global__ void __launch_bounds__(kPairAheadBlock, 6) k_dslash_mrhs_pair_ahead(c
     const int tile = blockIdx.x % a.ntiles;
     const int hh = (blockIdx.x / a.ntiles) * kPairAheadBlock + threadIdx.x;
     const bool valid = hh < a.Vh;
-    if ((EPI == 0 || EPI == 4) && !valid) return;  // (EPI 1-3: every thread takes part in the sums)
     const int h = valid ? hh : (int)a.Vh - 1;
     const int r0 = 2 * tile;
-    // restart hops (EPI 3, 4): a pair of retired RHS has nothing to compute (whole block)
-    if (EPI >= 3 && !a.sink.active[r0] && !(r0 + 1 < a.nrhs && a.sink.active[r0 + 1])) return;
     const bool two = r0 + 1 < a.nrhs;
     const char *in0 = a.in + (size_t)r0 * a.fbytes;
     const char *in1 = two ? in0 + a.fbytes : in0;
@@ -352,6 +350,10 @@ __global__ void __launch_bounds__(kPairAheadBlock, 6) k_dslash_mrhs_pair_ahead(c
     int nb[8];
     neighbour_sites(c, xh, a.L0, a.L0h, a.L1, a.L2, a.L3, nb);
     const f2 sg((float)a.g5_in);
+    pdl_start();
+    if ((EPI == 0 || EPI == 4) && !valid) return;  // (EPI 1-3: every thread takes part in the sums)
+    // restart hops (EPI 3, 4): a pair of retired RHS has nothing to compute (whole block)
+    if (EPI >= 3 && !a.sink.active[r0] && !(r0 + 1 < a.nrhs && a.sink.active[r0 + 1])) return;
     RawSpinor<SIO> ra[2], rb[2];
     RawLink<LIO> rl[2];
     auto issue = [&](int k) {
@@ -415,18 +417,21 @@ static int launch_pair(const Geom &g, cudaStream_t s, MrhsArgs a, bool ahead, in
         a.ntiles = (a.nrhs + 1) / 2;
         const long nblk = (g.Vh + block - 1) / block * a.ntiles;
         if (nblk > 0x7fffffffL) return set_error(PLQCD_ERR_ARG, "dslash_mrhs: grid too large");
-        auto k = ahead ? (epi == 4 ? k_dslash_mrhs_pair_ahead<SIO, LIO, false, 4>
-                        : epi == 3 ? k_dslash_mrhs_pair_ahead<SIO, LIO, true, 3>
-                        : epi == 2 ? k_dslash_mrhs_pair_ahead<SIO, LIO, true, 2>
-                        : epi == 1 ? k_dslash_mrhs_pair_ahead<SIO, LIO, true, 1>
-                        : xpay     ? k_dslash_mrhs_pair_ahead<SIO, LIO, true, 0>
-                                   : k_dslash_mrhs_pair_ahead<SIO, LIO, false, 0>)
-                       : (epi == 4 ? k_dslash_mrhs_pair<SIO, LIO, false, 4>
-                        : epi == 3 ? k_dslash_mrhs_pair<SIO, LIO, true, 3>
-                        : epi == 2 ? k_dslash_mrhs_pair<SIO, LIO, true, 2>
-                        : epi == 1 ? k_dslash_mrhs_pair<SIO, LIO, true, 1>
-                        : xpay     ? k_dslash_mrhs_pair<SIO, LIO, true, 0>
-                                   : k_dslash_mrhs_pair<SIO, LIO, false, 0>);
+        if (ahead) {
+            auto k = epi == 4 ? k_dslash_mrhs_pair_ahead<SIO, LIO, false, 4>
+                   : epi == 3 ? k_dslash_mrhs_pair_ahead<SIO, LIO, true, 3>
+                   : epi == 2 ? k_dslash_mrhs_pair_ahead<SIO, LIO, true, 2>
+                   : epi == 1 ? k_dslash_mrhs_pair_ahead<SIO, LIO, true, 1>
+                   : xpay     ? k_dslash_mrhs_pair_ahead<SIO, LIO, true, 0>
+                              : k_dslash_mrhs_pair_ahead<SIO, LIO, false, 0>;
+            return launch_overlapped(k, (unsigned)nblk, block, s, a);
+        }
+        auto k = epi == 4 ? k_dslash_mrhs_pair<SIO, LIO, false, 4>
+               : epi == 3 ? k_dslash_mrhs_pair<SIO, LIO, true, 3>
+               : epi == 2 ? k_dslash_mrhs_pair<SIO, LIO, true, 2>
+               : epi == 1 ? k_dslash_mrhs_pair<SIO, LIO, true, 1>
+               : xpay     ? k_dslash_mrhs_pair<SIO, LIO, true, 0>
+                          : k_dslash_mrhs_pair<SIO, LIO, false, 0>;
         k<<<(unsigned)nblk, block, 0, s>>>(a);
         PLQCD_CUDA_TRY(cudaGetLastError());
         return PLQCD_OK;
@@ -546,9 +551,9 @@ bool dslash_mrhs_tuned(const Geom &g, int prec, int recon, int nrhs, bool xpay) 
     return tune_lookup(key, nullptr);
 }
 
-// out (nrhs fields) = a_up/a_low * H in + b * x; tuned over RHS tile and block
-static int mrhs_args(const Geom &g, const void *gauge, int prec, void *out, const void *in, int nrhs,
-                     int out_parity, unsigned flags, double a, const void *x, double b, dev::MrhsArgs &m) {
+// out (nrhs fields) = a_up/a_low * H in + b * x
+int mrhs_args(const Geom &g, const void *gauge, int prec, void *out, const void *in, int nrhs, int out_parity,
+              unsigned flags, double a, const void *x, double b, dev::MrhsArgs &m) {
     if (nrhs < 1) return set_error(PLQCD_ERR_ARG, "dslash_mrhs: nrhs must be >= 1");
     PLQCD_TRY(check_field_ptr(out, "dslash_mrhs"));
     PLQCD_TRY(check_field_ptr(in, "dslash_mrhs"));

@@ -160,7 +160,7 @@ int launch_dslash_tma_mrhs(const Geom &g, cudaStream_t s, const void *gauge, int
                            double b, int kind, int nstage, int ny, int nr);
 // the device flag a TMA stage wait sets when it runs out (reset: clear it)
 int dslash_tma_status(bool reset);
-// variant 0: direct loads, 2/3: cp.async pipeline depth; no tuning
+// variant 0: loads ahead in registers, 2/3: cp.async pipeline depth; no tuning
 int launch_dslash_config(const Geom &g, cudaStream_t s, const DslashCall &c, int variant, int block);
 // nrhs one-parity fields back to back: out = a * H in (+ b * x if x != null)
 int launch_dslash_mrhs(const Geom &g, cudaStream_t s, const void *gauge, int prec, int recon, void *out,

@@ -40,6 +40,7 @@ namespace plqcd {
 
 struct McgState {  // device arrays of length nrhs, plus reduction scratch
     double *rr, *rr_old, *pAp, *alpha, *beta, *sr2, *bp2, *maxrr, *target, *aux;
+    double *check;  // |b - D x|^2 and |b|^2 of the even, then of the odd sites: 4 * nrhs
     int *active, *conv_iter;
     int *fresh;  // 1: the sloppy solution x_s was folded into x and counts as zero
     double *partials;  // nrhs * nb
@@ -143,24 +144,6 @@ __global__ void __launch_bounds__(kBlasBlock) k_mnorm2(const char *x, size_t fb,
         v += n2(s);
     }
     mreduce(v, st, op, tol2);
-}
-
-// out = a - b (F64) ; |out|^2 -> op
-__global__ void __launch_bounds__(kBlasBlock) k_msub_norm2(char *out, const char *a, const char *b, size_t fb,
-                                                           long Vh, McgState st, MOp op) {
-    const int f = blockIdx.y;
-    const size_t o = (size_t)f * fb;
-    double v = 0;
-    for (long h = (long)blockIdx.x * blockDim.x + threadIdx.x; h < Vh; h += (long)gridDim.x * blockDim.x) {
-        cx<double> av[12], bv[12];
-        SpinorIO<PLQCD_F64>::load(a + o, Vh, h, av);
-        SpinorIO<PLQCD_F64>::load(b + o, Vh, h, bv);
-#pragma unroll
-        for (int k = 0; k < 12; k++) av[k] = csub(av[k], bv[k]);
-        SpinorIO<PLQCD_F64>::store(out + o, Vh, h, av);
-        v += n2(av);
-    }
-    mreduce(v, st, op, 0.0);
 }
 
 // z = a - b (F64) ; |z|^2 -> op ; out = z in the sloppy format SP (the
@@ -414,7 +397,7 @@ struct Item {
     // the sloppy hops that produce t and Ap carry |t|^2 and r -= alpha Ap,
     // |r|^2 in their epilogues (RHS-pair kernels; see RhsSink)
     bool fused = false;
-    double *hop_partials = nullptr;  // nrhs * ceil(Vh / 32)
+    double *hop_partials = nullptr;  // 2 * nrhs * ceil(Vh / 32)
 };
 
 struct Batch {
@@ -489,13 +472,6 @@ struct Batch {
         PLQCD_CUDA_TRY(cudaGetLastError());
         return PLQCD_OK;
     }
-    int sub_norm2(Item &it, void *out, const void *a, const void *b, MOp op) {
-        dim3 grid(it.st.nb, it.in.nrhs);
-        dev::k_msub_norm2<<<grid, kBlasBlock, 0, s>>>((char *)out, (const char *)a, (const char *)b, it.fb64,
-                                                      it.g->Vh, it.st, op);
-        PLQCD_CUDA_TRY(cudaGetLastError());
-        return PLQCD_OK;
-    }
     int convert(Item &it, void *dst, int dp, const void *src, int sp) {
         dim3 grid(it.st.nb, it.in.nrhs);
         const size_t fd = spinor_parity_bytes(it.g->Vh, dp), fs = spinor_parity_bytes(it.g->Vh, sp);
@@ -512,6 +488,42 @@ struct Batch {
 #undef F
 #undef G
         PLQCD_CUDA_TRY(cudaGetLastError());
+        return PLQCD_OK;
+    }
+
+    // FP64: out (prec) = c - (x + a H in), its |.|^2 per RHS -> sums, in the
+    // hop's epilogue; with one RHS that kernel has no links to share, and the
+    // hop and the difference stay apart (tmp: F64 scratch)
+    int resid(Item &it, void *out, int prec, const void *in, const void *x, double a, const void *c, void *tmp) {
+        if (it.in.nrhs > 1) {
+            HopSum h;
+            h.kind = HOP_RESID;
+            h.c = c;
+            h.out_prec = prec;
+            return launch_mrhs_links_sum(*it.g, s, it.in.g64, out, in, it.in.nrhs, PLQCD_EVEN, a, x, 1.0, h,
+                                         it.hop_partials, it.st.sr2);
+        }
+        PLQCD_TRY(hop(it, it.in.g64, tmp, in, PLQCD_EVEN, 0, x, a, 1.0));
+        return sub_norm2_to(it, out, prec, c, tmp, M_SR2);
+    }
+    // |b - D x|^2 and |b|^2 per RHS of one parity -> st.check
+    int check(Item &it, int par) {
+        const void *xo = par ? it.in.x_even : it.in.x_odd, *xs_ = par ? it.in.x_odd : it.in.x_even;
+        const void *bb = par ? it.in.b_odd : it.in.b_even;
+        const int n = it.in.nrhs;
+        double *sums = it.st.check + 2 * n * par;
+        if (n > 1) {
+            HopSum h;
+            h.kind = HOP_CHECK;
+            h.c = bb;
+            return launch_mrhs_links_sum(*it.g, s, it.in.g64, it.t64, xo, n, par, -kappa, xs_, 1.0, h, it.hop_partials,
+                                         sums);
+        }
+        PLQCD_TRY(hop(it, it.in.g64, it.t64, xo, par, 0, xs_, -kappa, 1.0));
+        PLQCD_TRY(sub_norm2_to(it, it.r64, PLQCD_F64, bb, it.t64, M_AUX));
+        PLQCD_CUDA_TRY(cudaMemcpyAsync(sums, it.st.aux, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
+        PLQCD_TRY(norm2(it, bb, PLQCD_F64, M_AUX, false));
+        PLQCD_CUDA_TRY(cudaMemcpyAsync(sums + n, it.st.aux, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
         return PLQCD_OK;
     }
 
@@ -539,13 +551,13 @@ struct Batch {
         for (Item &it : items) {
             PLQCD_TRY(accum(it, true));
             // FP64: solution and Schur residual b' - Mhat x (convergence)
-            PLQCD_TRY(mhat(it, it.in.g64, it.t64, it.in.x_even, it.tmp64, false));
+            PLQCD_TRY(hop(it, it.in.g64, it.tmp64, it.in.x_even, PLQCD_ODD, 0));
             // restart direction Mhat^dag r: the sloppy operator's accuracy
             // suffices (FP64 when the solve is FP64), so the mixed solve
             // writes r only in the sloppy format
             if (mixed) {
                 const plqcd_gauge *gs = it.in.g_sloppy ? it.in.g_sloppy : it.in.g64;
-                PLQCD_TRY(sub_norm2_to(it, it.t, it.ps, it.bprime, it.t64, M_SR2));
+                PLQCD_TRY(resid(it, it.t, it.ps, it.tmp64, it.in.x_even, -kappa * kappa, it.bprime, it.t64));
                 PLQCD_TRY(ctl_converged(it));
                 if (it.fused) {
                     // |r|^2 in the second hop; pairs of retired RHS skipped
@@ -555,7 +567,7 @@ struct Batch {
                     PLQCD_TRY(norm2(it, it.rs, it.ps, M_RR_TRUE, false));
                 }
             } else {
-                PLQCD_TRY(sub_norm2(it, it.r64, it.bprime, it.t64, M_SR2));
+                PLQCD_TRY(resid(it, it.r64, PLQCD_F64, it.tmp64, it.in.x_even, -kappa * kappa, it.bprime, it.t64));
                 PLQCD_TRY(ctl_converged(it));
                 PLQCD_TRY(mhat(it, it.in.g64, it.t64, it.r64, it.tmp64, true));
                 PLQCD_TRY(norm2(it, it.t64, PLQCD_F64, M_RR_TRUE, false));
@@ -619,7 +631,7 @@ int alloc_item(Batch &B, Item &it, bool own_ws, int nitems) {
     const size_t nsb = (size_t)(Vh + 31) / 32;  // site blocks of a fused hop, at most
     const size_t need = 4 * al(it.fb64 * n) + 5 * al(it.fbs * n) + al(it.fbx * n) + 10 * al(sizeof(double) * n) +
                         3 * al(sizeof(int) * n) + al(sizeof(double) * n * it.st.nb) + al(sizeof(unsigned) * n) +
-                        al(sizeof(double) * n * nsb) + al(sizeof(McgControl)) + al(sizeof(McgState) * nitems);
+                        al(sizeof(double) * 2 * n * nsb) + al(sizeof(double) * 4 * n) + al(sizeof(McgControl)) + al(sizeof(McgState) * nitems);
     void *ws = nullptr;
     if (own_ws) {
         if (cudaMalloc(&it.mem, need) != cudaSuccess) {
@@ -654,7 +666,8 @@ int alloc_item(Batch &B, Item &it, bool own_ws, int nitems) {
     it.st.fresh = reinterpret_cast<int *>(take(sizeof(int) * n));
     it.st.partials = reinterpret_cast<double *>(take(sizeof(double) * n * it.st.nb));
     it.st.counters = reinterpret_cast<unsigned *>(take(sizeof(unsigned) * n));
-    it.hop_partials = reinterpret_cast<double *>(take(sizeof(double) * n * nsb));
+    it.hop_partials = reinterpret_cast<double *>(take(sizeof(double) * 2 * n * nsb));
+    it.st.check = reinterpret_cast<double *>(take(sizeof(double) * 4 * n));
     // the first item's workspace also holds the batch's control block and states
     if (!B.ctl) B.ctl = reinterpret_cast<McgControl *>(take(sizeof(McgControl)));
     if (!B.st_dev) B.st_dev = reinterpret_cast<McgState *>(take(sizeof(McgState) * nitems));
@@ -688,6 +701,7 @@ int tune_item(Batch &B, Item &it) {
     const plqcd_solve_item &in = it.in;
     const plqcd_gauge *gs = in.g_sloppy ? in.g_sloppy : in.g64;
     const int n = in.nrhs;
+    if (n > 1) PLQCD_TRY(preload_mrhs_links_resid(in.g64->recon, B.mixed ? it.ps : PLQCD_F64));
     const bool done = dslash_mrhs_tuned(*it.g, gs->prec, gs->recon, n, false) &&
                       dslash_mrhs_tuned(*it.g, gs->prec, gs->recon, n, true) &&
                       dslash_mrhs_tuned(*it.g, PLQCD_F64, in.g64->recon, n, false) &&
@@ -969,28 +983,17 @@ extern "C" int plqcd_invert_cg_batch(plqcd_solve_item *items, int nitems, const 
         inf.converged = 1;
         for (Item &it : B.items) {
             const int n = it.in.nrhs;
-            std::vector<double> r2(n, 0.0), b2(n, 0.0), tmp(n), sr2(n), bp2(n);
-            std::vector<int> act(n), conv(n);
-            for (int par = 0; par < 2 && rc == PLQCD_OK; par++) {
-                const void *xo = par ? it.in.x_even : it.in.x_odd, *xs_ = par ? it.in.x_odd : it.in.x_even;
-                const void *bb = par ? it.in.b_odd : it.in.b_even;
-                if ((rc = B.hop(it, it.in.g64, it.t64, xo, par, 0, xs_, -B.kappa, 1.0))) break;
-                if ((rc = B.sub_norm2(it, it.r64, bb, it.t64, M_AUX))) break;
-                cudaMemcpyAsync(tmp.data(), it.st.aux, sizeof(double) * n, cudaMemcpyDeviceToHost, B.s);
-                cudaStreamSynchronize(B.s);
-                for (int f = 0; f < n; f++) r2[f] += tmp[f];
-                if ((rc = B.norm2(it, bb, PLQCD_F64, M_AUX, false))) break;
-                cudaMemcpyAsync(tmp.data(), it.st.aux, sizeof(double) * n, cudaMemcpyDeviceToHost, B.s);
-                cudaStreamSynchronize(B.s);
-                for (int f = 0; f < n; f++) b2[f] += tmp[f];
-            }
-            if (rc) break;
+            std::vector<double> chk(4 * n), sr2(n), bp2(n);
+            std::vector<int> act(n);
+            if ((rc = B.check(it, PLQCD_EVEN)) || (rc = B.check(it, PLQCD_ODD))) break;
+            cudaMemcpyAsync(chk.data(), it.st.check, sizeof(double) * 4 * n, cudaMemcpyDeviceToHost, B.s);
             cudaMemcpyAsync(sr2.data(), it.st.sr2, sizeof(double) * n, cudaMemcpyDeviceToHost, B.s);
             cudaMemcpyAsync(bp2.data(), it.st.bp2, sizeof(double) * n, cudaMemcpyDeviceToHost, B.s);
             cudaMemcpyAsync(act.data(), it.st.active, sizeof(int) * n, cudaMemcpyDeviceToHost, B.s);
             cudaStreamSynchronize(B.s);
             for (int f = 0; f < n; f++) {
-                const double tr = b2[f] > 0 ? sqrt(r2[f] / b2[f]) : 0.0;
+                const double r2 = chk[f] + chk[2 * n + f], b2 = chk[n + f] + chk[3 * n + f];
+                const double tr = b2 > 0 ? sqrt(r2 / b2) : 0.0;
                 const double sr = bp2[f] > 0 ? sqrt(sr2[f] / bp2[f]) : 0.0;
                 if (true_residuals) true_residuals[off + f] = tr;
                 inf.max_true_residual = std::max(inf.max_true_residual, tr);

@@ -4,6 +4,7 @@
 
 #include "dslash_core.cuh"
 #include "internal.h"
+#include "raw_loads.cuh"
 
 namespace plqcd {
 namespace dev {
@@ -65,7 +66,7 @@ __device__ __forceinline__ void pair_epilogue(const MrhsArgs &a, int r0, bool tw
                 const float al = (float)a.sink.alpha[f];
                 char *rf = a.sink.rvec + (size_t)f * a.fbytes;
                 cx<float> rv[12];
-                SIO::load(rf, a.Vh, h, rv);
+                load_coherent<SIO>(rf, a.Vh, h, rv);
 #pragma unroll
                 for (int k = 0; k < 12; k++) rv[k] = {fmaf(-al, o[k].re, rv[k].re), fmaf(-al, o[k].im, rv[k].im)};
                 SIO::store(rf, a.Vh, h, rv);
@@ -79,4 +80,9 @@ __device__ __forceinline__ void pair_epilogue(const MrhsArgs &a, int r0, bool tw
 }
 
 }  // namespace dev
+
+// checked arguments of a multi-RHS launch (dslash_mrhs.cu)
+int mrhs_args(const Geom &g, const void *gauge, int prec, void *out, const void *in, int nrhs, int out_parity,
+              unsigned flags, double a, const void *x, double b, dev::MrhsArgs &m);
+
 }  // namespace plqcd
