@@ -328,7 +328,9 @@ extern "C" int plqcd_tune_count(void) {
 
 extern "C" int plqcd_tune_get(const char *key, int *variant, int *block, double *ms) {
     plqcd::TuneResult r;
-    if (!key || !plqcd::tune_lookup(key, &r)) return plqcd::set_error(PLQCD_ERR_ARG, "tune: no entry for key");
+    // (a key without its candidate list's number names the launch: its entry of the present list first)
+    if (!key || (!plqcd::tune_lookup(std::string(key) + "|c2", &r) && !plqcd::tune_lookup(key, &r)))
+        return plqcd::set_error(PLQCD_ERR_ARG, "tune: no entry for key");
     if (variant) *variant = r.variant;
     if (block) *block = r.block;
     if (ms) *ms = r.ms;
