@@ -307,7 +307,9 @@ def kernel_name(cfg) -> str:
         return f"k_dslash_tma<F64,18> ({(v // 100) % 10} stages, {v % 100} rows per tile, full lattice)"
     if v in (2, 3):
         return f"k_dslash_pipe<F64,18,full> (depth {v}, block {b})"
-    return f"k_dslash<F64,18,full> (block {b})"
+    if v == 21:
+        return f"k_dslash_ahead<F64,18,full> (parities joined, 2x2x2 tiles)"
+    return f"k_dslash_ahead<F64,18,full> (depth {2 if b == 128 else 1})"
 
 
 def time_kernel(torch, fn, steps: int, warmup: int, d: Dist | None = None):
