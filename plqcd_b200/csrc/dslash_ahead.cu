@@ -159,7 +159,6 @@ template <class SIO, class LIO, int MODE, int DEPTH, int MINB, int SUM = 0, int 
 __global__ void __launch_bounds__(kAheadBlock, MINB) k_dslash_ahead(const DslashArgs a, const SumArgs q) {
     using R = typename SIO::real;
     static_assert(SUM == 0 || MODE == 1, "sums belong to the xpay epilogue");
-    if (a.halt && *a.halt) return;
     constexpr bool XPAY = MODE == 1, FULL = MODE >= 2;
     int par;
     long h;
@@ -200,7 +199,7 @@ __global__ void __launch_bounds__(kAheadBlock, MINB) k_dslash_ahead(const Dslash
     int nb[8];
     neighbour_sites(c, xh, a.L0, a.L0h, a.L1, a.L2, a.L3, nb);
     pdl_start();
-    if (a.halt && *a.halt) return;
+    if (a.halt && *a.halt) return;  // (an earlier kernel writes the flag: never read ahead of the wait)
 
     constexpr int S = DEPTH + 1;
     RawSpinor<SIO> rs[S];
