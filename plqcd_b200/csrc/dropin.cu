@@ -33,9 +33,15 @@ namespace {
 // t-slab chunks of the copy/compute pipeline (chunk_plan)
 constexpr int kMaxChunks = 64;
 
-struct SplitCache {  // gauge field of the split entry points, by host address
-    const double *re = nullptr, *im = nullptr;
+// what a device copy of the links was loaded from. `dirty`: nothing, or an
+// array declared changed since (plqcd_gauge_update marks every copy; only the
+// copy's own upload clears the mark)
+struct LinkCache {
+    const void *u = nullptr;   // host array (split family: its real plane)
+    const void *im = nullptr;  // split family: the imaginary plane
+    int lanes = 0;             // lane-packed family
     uint64_t fp = 0;
+    bool dirty = true;
 };
 
 // what a captured pipeline graph depends on besides the device buffers
@@ -53,8 +59,7 @@ constexpr int kGraphSlots = 4;
 
 struct DropIn {
     plqcd_gauge *gauge_split = nullptr, *gauge12 = nullptr;
-    SplitCache split18, split12;
-    bool dirty_split = true;
+    LinkCache split18, split12;
     int dims[4] = {0, 0, 0, 0};
     cudaStream_t s_h2d = nullptr, s_d2h = nullptr;  // copy streams
     cudaEvent_t ev_in[kMaxChunks] = {}, ev_out[kMaxChunks] = {}, ev_k0[kMaxChunks] = {}, ev_k1[kMaxChunks] = {};
@@ -62,9 +67,7 @@ struct DropIn {
     plqcd_gauge *gauge = nullptr;
     void *aos_in = nullptr, *aos_out = nullptr;  // API layout staging, one parity
     void *f_in = nullptr, *f_out = nullptr;      // kernel layout (F64), one parity
-    const su3 *cached_u = nullptr;
-    uint64_t fingerprint = 0;
-    bool dirty = true;
+    LinkCache links;                             // of `gauge`
     cudaStream_t stream = nullptr;  // owned by the drop-in path
     double kernel_ms = 0, h2d = 0, d2h = 0;
     cudaEvent_t ev_fork = nullptr, ev_join[2] = {nullptr, nullptr};  // capture fork / join
@@ -75,12 +78,7 @@ struct DropIn {
     bool last_valid = false;
     // lane-packed entry points (spinor_256 / spinor_512 and su3_256 / su3_512)
     plqcd_gauge *gauge_packed = nullptr, *gauge_packed12 = nullptr;
-    struct {
-        const void *u = nullptr;
-        int lanes = 0;
-        uint64_t fp = 0;
-    } packed18, packed12;
-    bool dirty_packed = true;
+    LinkCache packed18, packed12;
 };
 
 std::mutex g_mu;
@@ -175,35 +173,34 @@ uint64_t fingerprint(const su3 *u, long nlinks) {
     return h;
 }
 
-// Whether the device copy of link array `u` (cached from the array at
-// `cached`, with sampled fingerprint `cached_fp`) can serve this call:
+// Whether the device copy `c` of link array `u` can serve this call:
 //   PLQCD_GAUGE_CACHE unset: only a registered array, not marked dirty;
 //   PLQCD_GAUGE_CACHE=1:     any array whose address and fingerprint match;
 //   PLQCD_GAUGE_CACHE=0:     never.
 // `fp` computes the fingerprint (only the sampled mode needs it).
 template <class F>
-bool keep_cached_gauge(const void *u, const void *cached, bool dirty, uint64_t cached_fp, uint64_t *new_fp, F fp) {
+bool keep_cached_gauge(const void *u, const LinkCache &c, uint64_t *new_fp, F fp) {
     const char *e = getenv("PLQCD_GAUGE_CACHE");
     if (e && *e == '0') return false;
     if (e && *e && *e != '0') {
         *new_fp = fp();
-        return !dirty && cached == u && cached_fp == *new_fp;
+        return !c.dirty && c.u == u && c.fp == *new_fp;
     }
-    return !dirty && cached == u && g_registered == u;
+    return !c.dirty && c.u == u && g_registered == u;
 }
 
 // A call queues the upload of its links and waits once, at its end. A call
 // that fails on the way waits as well (the caller gets its arrays back) and
-// marks the device copy of the links as not loaded.
+// marks the device copy of the links it uses as not loaded.
 struct CallGuard {
-    bool &dirty;
+    LinkCache &links;
     bool ok = false;
     ~CallGuard() {
         if (ok) return;
         for (cudaStream_t st : {g_d.s_h2d, g_d.s_d2h, g_d.stream})
             if (st) cudaStreamSynchronize(st);
         cudaGetLastError();
-        dirty = true;
+        links.dirty = true;
     }
 };
 
@@ -251,7 +248,6 @@ int ensure_locked() {
         release_locked();
         return set_error(PLQCD_ERR_CUDA, "drop-in: stream/event creation failed");
     }
-    g_d.dirty = true;
     return PLQCD_OK;
 }
 
@@ -403,15 +399,16 @@ double hop_call(spinor *qin, spinor *qout, su3 *u, int out_parity) {
         return -1.0;
     }
     g_d.h2d = g_d.d2h = 0;
-    CallGuard guard{g_d.dirty};
+    LinkCache &lc = g_d.links;
+    CallGuard guard{lc};
 
     // gauge field: upload unless the device copy may serve (keep_cached_gauge)
     uint64_t fp = 0;
-    if (!keep_cached_gauge(u, g_d.cached_u, g_d.dirty, g_d.fingerprint, &fp, [&] { return fingerprint(u, 8 * Vh); })) {
+    if (!keep_cached_gauge(u, lc, &fp, [&] { return fingerprint(u, 8 * Vh); })) {
         if (upload_links(g_d.gauge, u) != PLQCD_OK) return -1.0;
-        g_d.cached_u = u;
-        g_d.fingerprint = fp;
-        g_d.dirty = false;
+        lc.u = u;
+        lc.fp = fp;
+        lc.dirty = false;
         g_d.h2d += 8.0 * Vh * sizeof(su3);
     }
 
@@ -521,21 +518,21 @@ double hop_call_split(double *qout_re, double *qout_im, double *u_re, double *u_
         return -1.0;
     }
     g_d.h2d = g_d.d2h = 0;
-    CallGuard guard{g_d.dirty_split};
+    LinkCache &lc = short12 ? g_d.split12 : g_d.split18;
+    CallGuard guard{lc};
     plqcd_gauge *&gf = short12 ? g_d.gauge12 : g_d.gauge_split;
     if (!gf && plqcd_gauge_create(lat, PLQCD_F64, short12 ? 12 : 18, &gf) != PLQCD_OK) return -1.0;
-    SplitCache &sc = short12 ? g_d.split12 : g_d.split18;
     uint64_t fp = 0;
     // the split family registers its real-part plane u_re
-    if (sc.im != u_im ||
-        !keep_cached_gauge(u_re, sc.re, g_d.dirty_split, sc.fp, &fp, [&] { return fingerprint_split(u_re, u_im, 8 * Vh * 9); })) {
+    if (lc.im != u_im ||
+        !keep_cached_gauge(u_re, lc, &fp, [&] { return fingerprint_split(u_re, u_im, 8 * Vh * 9); })) {
         if (load_gauge_split(gf, u_re, u_im) != PLQCD_OK) return -1.0;
-        sc.re = u_re;
-        sc.im = u_im;
-        sc.fp = fp;
+        lc.u = u_re;
+        lc.im = u_im;
+        lc.fp = fp;
+        lc.dirty = false;
         g_d.h2d += 2.0 * sizeof(double) * 9 * 8 * Vh;
     }
-    g_d.dirty_split = false;
     const int in_parity = out_parity ^ 1;
     const size_t half = sizeof(double) * 12 * Vh;
     double *dre = static_cast<double *>(g_d.aos_in), *dim = dre + 12 * Vh;
@@ -660,21 +657,20 @@ double hop_call_packed(const void *qin, void *qout, const void *u, int out_parit
         return -1.0;
     }
     g_d.h2d = g_d.d2h = 0;
-    CallGuard guard{g_d.dirty_packed};
+    LinkCache &lc = short12 ? g_d.packed12 : g_d.packed18;
+    CallGuard guard{lc};
     plqcd_gauge *&gf = short12 ? g_d.gauge_packed12 : g_d.gauge_packed;
     if (!gf && plqcd_gauge_create(lat, PLQCD_F64, short12 ? 12 : 18, &gf) != PLQCD_OK) return -1.0;
-    auto &pc = short12 ? g_d.packed12 : g_d.packed18;
     uint64_t fp = 0;
-    if (pc.lanes != lanes || !keep_cached_gauge(u, pc.u, g_d.dirty_packed, pc.fp, &fp, [&] {
-            return fingerprint(static_cast<const su3 *>(u), 8 * Vh);
-        })) {
+    if (lc.lanes != lanes ||
+        !keep_cached_gauge(u, lc, &fp, [&] { return fingerprint(static_cast<const su3 *>(u), 8 * Vh); })) {
         if (load_gauge_packed(gf, u, lanes) != PLQCD_OK) return -1.0;
-        pc.u = u;
-        pc.lanes = lanes;
-        pc.fp = fp;
+        lc.u = u;
+        lc.lanes = lanes;
+        lc.fp = fp;
+        lc.dirty = false;
         g_d.h2d += 8.0 * Vh * sizeof(su3);
     }
-    g_d.dirty_packed = false;
     const int in_parity = out_parity ^ 1;
     const size_t half = sizeof(spinor) * Vh;  // one parity, in either layout
     void *stage = g_d.aos_out, *aos = g_d.aos_in;
@@ -729,9 +725,7 @@ void dropin_release() {
 extern "C" int plqcd_gauge_update(const su3 *u) {
     std::lock_guard<std::mutex> lk(g_mu);
     g_registered = u;
-    g_d.dirty = true;
-    g_d.dirty_split = true;
-    g_d.dirty_packed = true;
+    for (LinkCache *c : {&g_d.links, &g_d.split18, &g_d.split12, &g_d.packed18, &g_d.packed12}) c->dirty = true;
     return PLQCD_OK;
 }
 
