@@ -190,11 +190,13 @@ static int launch_pipe(const Geom &g, cudaStream_t s, const DslashArgs &a, int b
 
 // variant 2, 3: cp.async pipeline of that depth; anything else: loads ahead
 // in registers (0 and 21 of dslash_ahead.cu; tuning files may still hold 12
-// and 13, kernels that it replaced)
+// and 13, kernels of two sites per thread that it replaced where they existed)
 template <class SIO, class LIO, bool COMPAT, bool XPAY, bool FULL>
 static int launch_t(const Geom &g, cudaStream_t s, const DslashArgs &a, int prec, int recon, int variant, int block) {
     if (variant == 2) return launch_pipe<SIO, LIO, 2, COMPAT, XPAY, FULL>(g, s, a, block);
     if (variant == 3) return launch_pipe<SIO, LIO, 3, COMPAT, XPAY, FULL>(g, s, a, block);
+    if ((variant == 12 || variant == 13) && (COMPAT || FULL || std::is_same<typename SIO::real, double>::value))
+        return set_error(PLQCD_ERR_ARG, "dslash: two sites per thread exists for 32/16-bit single-parity calls");
     if constexpr (COMPAT) {
         const long nblk = (a.h_end - a.h_begin + block - 1) / block * a.nrhs;
         k_dslash_compat<SIO, LIO><<<(unsigned)nblk, block, 0, s>>>(a);

@@ -134,3 +134,33 @@ def test_dependent_launches_back_to_back(cuda, monkeypatch, dims, prec, recon):
         lat.synchronize()
         got.append(a)
     assert bool((got[0] == got[1]).all()) and bool((got[0] == got[2]).all())
+
+
+@pytest.mark.parametrize("variant", [12, 13])
+def test_two_site_numbers_refuse_what_they_refused(cuda, monkeypatch, variant):
+    """12 and 13 stood for kernels of two sites per thread, which existed for
+    one parity in 32 and 16 bits: there the numbers still run, elsewhere they
+    are an error."""
+    lat = new_lattice((4, 4, 4, 4))
+    _force(monkeypatch, variant, 64)
+    monkeypatch.setenv("PLQCD_MRHS_VARIANT", str(100 + variant))
+    monkeypatch.setenv("PLQCD_MRHS_BLOCK", "64")
+    for prec, recon in FORMATS:
+        g = P.Gauge(lat, prec, recon)
+        g.random(1)
+        nb = lat.spinor_bytes(prec)
+        a, b, c, d = (dev_bytes(nb) for _ in range(4))
+        lat.spinor_gaussian(a, prec, 0, 2)
+        lat.spinor_gaussian(b, prec, 1, 3)
+        one = [lambda: lat.dslash(g, c, b, 0, prec), lambda: lat.dslash_xpay(g, c, b, 0, prec, 0.5, a, 1.0),
+               lambda: lat.dslash_mrhs(g, c, b, 1, 0, prec)]
+        refused = [lambda: lat.dslash_full(g, c, d, a, b, prec)]
+        if prec == P.F64:
+            refused += one + ([lambda: lat.dslash(g, c, b, 0, prec, P.DSLASH_COMPAT)] if recon == 18 else [])
+        else:
+            for call in one:
+                call()
+        for call in refused:
+            with pytest.raises(P.PlqcdError, match="two sites per thread"):
+                call()
+    lat.synchronize()
