@@ -136,6 +136,36 @@ def test_dependent_launches_back_to_back(cuda, monkeypatch, dims, prec, recon):
     assert bool((got[0] == got[1]).all()) and bool((got[0] == got[2]).all())
 
 
+@pytest.mark.parametrize("nrhs", [2, 3])
+@pytest.mark.parametrize("prec,recon,variant", [(P.F64, 18, 4202), (P.F64, 12, 4204), (P.F32, 18, 2200),
+                                                (P.F16, 12, 2200), (P.BF16, 12, 2200)])
+@pytest.mark.parametrize("dims", [(2, 2, 2, 2), (4, 6, 8, 10), (16, 16, 16, 16)])
+def test_dependent_multi_rhs_launches_back_to_back(cuda, monkeypatch, dims, prec, recon, variant, nrhs):
+    """The same chain with the multi-RHS kernels that overlap their predecessor."""
+    lat = new_lattice(dims)
+    g = P.Gauge(lat, prec, recon)
+    g.random(3)
+    nb = lat.spinor_bytes(prec)
+    start = dev_bytes(nrhs * nb)
+    for r in range(nrhs):
+        lat.spinor_gaussian(start[r * nb:], prec, 0, 8 + r)
+    monkeypatch.setenv("PLQCD_MRHS_VARIANT", str(variant))
+    monkeypatch.setenv("PLQCD_MRHS_BLOCK", "64")
+    got = []
+    for wait in (True, False, False):
+        a, b = start.clone(), dev_bytes(nrhs * nb)
+        for k in range(40):
+            lat.dslash_mrhs(g, b, a, nrhs, 1, prec)
+            if wait:
+                lat.synchronize()
+            lat.dslash_mrhs_xpay(g, a, b, nrhs, 0, prec, -0.01, a, 1.0)  # x is overwritten in place
+            if wait:
+                lat.synchronize()
+        lat.synchronize()
+        got.append(a)
+    assert bool((got[0] == got[1]).all()) and bool((got[0] == got[2]).all())
+
+
 @pytest.mark.parametrize("variant", [12, 13])
 def test_two_site_numbers_refuse_what_they_refused(cuda, monkeypatch, variant):
     """12 and 13 stood for kernels of two sites per thread, which existed for
