@@ -166,6 +166,35 @@ def test_dependent_multi_rhs_launches_back_to_back(cuda, monkeypatch, dims, prec
     assert bool((got[0] == got[1]).all()) and bool((got[0] == got[2]).all())
 
 
+@pytest.mark.parametrize("dims", DIMS)
+@pytest.mark.parametrize("prec,recon", [(P.F32, 18), (P.F32, 12), (P.F16, 12), (P.BF16, 12)])
+def test_packed_lanes_same_bits_as_scalar(cuda, monkeypatch, dims, prec, recon):
+    """Packed FP32 lanes round as scalar FP32 does: the kernels that compute on
+    them (two components of one site, or two right-hand sides) against the
+    scalar arithmetic of the RHS-tile kernel."""
+    lat = new_lattice(dims)
+    g = P.Gauge(lat, prec, recon)
+    g.random(13)
+    nb = lat.spinor_bytes(prec)
+    f, x = dev_bytes(2 * nb), dev_bytes(2 * nb)
+    for r in range(2):
+        lat.spinor_gaussian(f[r * nb:], prec, 1, 60 + r)
+        lat.spinor_gaussian(x[r * nb:], prec, 0, 80 + r)
+    flags = P.DSLASH_G5_IN | P.DSLASH_G5_OUT
+    got = {}
+    # 1: scalar, a thread per RHS; 100, 102, 103: the single-RHS kernels per RHS; 2200, 2102: RHS pairs
+    for v, block in [(1, 64), (100, 64), (100, 128), (102, 64), (103, 64), (2200, 64), (2102, 64)]:
+        monkeypatch.setenv("PLQCD_MRHS_VARIANT", str(v))
+        monkeypatch.setenv("PLQCD_MRHS_BLOCK", str(block))
+        o = [dev_bytes(2 * nb).fill_(7) for _ in range(2)]
+        lat.dslash_mrhs(g, o[0], f, 2, 0, prec)
+        lat.dslash_mrhs_xpay(g, o[1], f, 2, 0, prec, 0.25, x, -2.0, flags)
+        lat.synchronize()
+        got[v, block] = o
+    for v, o in got.items():
+        assert bool((o[0] == got[1, 64][0]).all()) and bool((o[1] == got[1, 64][1]).all()), v
+
+
 @pytest.mark.parametrize("variant", [12, 13])
 def test_two_site_numbers_refuse_what_they_refused(cuda, monkeypatch, variant):
     """12 and 13 stood for kernels of two sites per thread, which existed for
