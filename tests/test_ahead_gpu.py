@@ -223,3 +223,24 @@ def test_two_site_numbers_refuse_what_they_refused(cuda, monkeypatch, variant):
             with pytest.raises(P.PlqcdError, match="two sites per thread"):
                 call()
     lat.synchronize()
+
+
+@pytest.mark.parametrize("dims", DIMS)
+def test_compat_configurations_same_bits(cuda, monkeypatch, dims):
+    """Every configuration that the tuner tries for the bug-compatible hop."""
+    lat = new_lattice(dims)
+    g = P.Gauge(lat, P.F64, 18)
+    g.random(19)
+    nb = lat.spinor_bytes(P.F64)
+    f = [dev_bytes(nb) for _ in range(2)]
+    for par in (0, 1):
+        lat.spinor_gaussian(f[par], P.F64, par, 90 + par)
+    got = {}
+    for v in [(2, 64), (2, 128), (2, 256), (0, 64), (0, 128), (0, 256), (3, 64), (3, 128)]:
+        _force(monkeypatch, *v)
+        got[v] = [dev_bytes(nb).fill_(7) for _ in range(2)]
+        for par in (0, 1):
+            lat.dslash(g, got[v][par], f[1 - par], par, P.F64, P.DSLASH_COMPAT)
+        lat.synchronize()
+    for v, o in got.items():
+        assert bool((o[0] == got[2, 64][0]).all()) and bool((o[1] == got[2, 64][1]).all()), v
