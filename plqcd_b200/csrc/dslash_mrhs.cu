@@ -604,13 +604,13 @@ static bool mrhs_sink_config(const Geom &g, int prec, int recon, int nrhs, TuneR
     return true;
 }
 
-bool dslash_mrhs_sink_ok(const Geom &g, int prec, int recon, int nrhs, int *variant, int *block) {
+bool dslash_mrhs_sink_ok(const Geom &g, int prec, int recon, int nrhs, int config[4]) {
     TuneResult t, tp;
     if (prec == PLQCD_F64 || nrhs < 2 || !mrhs_sink_config(g, prec, recon, nrhs, &t) ||
         !mrhs_sink_config(g, prec, recon, nrhs, &tp, false))
         return false;
-    if (variant) *variant = t.variant;
-    if (block) *block = t.block;
+    const int c[4] = {t.variant, t.block, tp.variant, tp.block};
+    std::copy(c, c + 4, config);
     return true;
 }
 

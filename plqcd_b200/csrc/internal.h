@@ -185,8 +185,9 @@ struct RhsSink {
     char *rvec;
 };
 // launch_dslash_mrhs_sink can run this multi-RHS hop (it is tuned, and not
-// forced to another kernel than an RHS-pair one)
-bool dslash_mrhs_sink_ok(const Geom &g, int prec, int recon, int nrhs, int *variant = nullptr, int *block = nullptr);
+// forced to another kernel than an RHS-pair one). config: variant and block of
+// the xpay and of the plain form, which may run different kernels
+bool dslash_mrhs_sink_ok(const Geom &g, int prec, int recon, int nrhs, int config[4]);
 int launch_dslash_mrhs_sink(const Geom &g, cudaStream_t s, const void *gauge, int prec, int recon, void *out,
                             const void *in, int nrhs, int out_parity, unsigned flags, double a, const void *x,
                             double b, int epi, const RhsSink &sink);

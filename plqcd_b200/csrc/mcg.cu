@@ -682,14 +682,14 @@ int alloc_item(Batch &B, Item &it, bool own_ws, int nitems) {
 
 // true the first time a (CUDA context, lattice, format, RHS count, kernel
 // configuration) runs the fused hops in this process
-bool first_fused_use(const Geom &g, int prec, int recon, int nrhs, int variant, int block) {
+bool first_fused_use(const Geom &g, int prec, int recon, int nrhs, const int config[4]) {
     static std::mutex mu;
     static std::set<std::string> seen;
     const unsigned long long ctx = current_context_id();
     if (!ctx) return true;  // no context ID: warm every time
     char key[160];
-    snprintf(key, sizeof key, "%llu|%d|%d|%d|%dx%dx%dx%d|%d|%d", ctx, prec, recon, nrhs, g.L[0], g.L[1], g.L[2],
-             g.L[3], variant, block);
+    snprintf(key, sizeof key, "%llu|%d|%d|%d|%dx%dx%dx%d|%d|%d|%d|%d", ctx, prec, recon, nrhs, g.L[0], g.L[1], g.L[2],
+             g.L[3], config[0], config[1], config[2], config[3]);
     std::lock_guard<std::mutex> lk(mu);
     return seen.insert(key).second;
 }
@@ -713,16 +713,16 @@ int tune_item(Batch &B, Item &it) {
         PLQCD_TRY(B.mhat(it, gs, it.t, it.p, it.tmps, false));
         PLQCD_TRY(B.mhat(it, in.g64, it.t64, it.r64, it.tmp64, false));
     }
-    // fused CG sums when the tuned sloppy xpay hop is an RHS-pair kernel
-    // (PLQCD_MCG_FUSED=0: separate passes)
+    // fused CG sums in the sloppy RHS-pair hops (PLQCD_MCG_FUSED=0: separate
+    // passes)
     const char *e = getenv("PLQCD_MCG_FUSED");
-    int variant = 0, block = 0;
+    int config[4] = {};
     it.fused = B.mixed && !(e && e[0] == '0') &&
-               dslash_mrhs_sink_ok(*it.g, gs->prec, gs->recon, n, &variant, &block);
-    if (it.fused && first_fused_use(*it.g, gs->prec, gs->recon, n, variant, block)) {
-        // load the fused kernels and set their shared memory before any
-        // capture, once per device and configuration (on zeroed fields; the
-        // solve's start overwrites every scalar they set)
+               dslash_mrhs_sink_ok(*it.g, gs->prec, gs->recon, n, config);
+    if (it.fused && first_fused_use(*it.g, gs->prec, gs->recon, n, config)) {
+        // load the fused kernels before any capture, once per device and
+        // configuration (on zeroed fields; the solve's start overwrites every
+        // scalar they set)
         PLQCD_CUDA_TRY(cudaMemsetAsync(it.p, 0, it.fbs * n, B.s));
         PLQCD_CUDA_TRY(cudaMemsetAsync(it.rs, 0, it.fbs * n, B.s));
         PLQCD_TRY(B.mhat_fused(it, gs, it.t, it.p, it.tmps, false, 1));

@@ -2,6 +2,8 @@
 one CUDA-graph launch: every RHS must reach the FP64 residual and agree with
 the single-RHS solver; residuals are re-checked on the host with the
 oracle's full-lattice operator."""
+import json
+
 import numpy as np
 import pytest
 
@@ -117,3 +119,33 @@ def test_batch_fused_sums_match_separate_passes(cuda, monkeypatch, tmp_path, var
             assert np.linalg.norm(a - b) / np.linalg.norm(b) < 1e-8
     finally:
         P.lib().plqcd_tune_clear()
+
+
+def test_plain_hop_retuned_alone(cuda, tmp_path):
+    """The fused restart takes its first hop from the plain form's tuned
+    configuration: when only that one changes between two solves in one graph
+    each, the kernel it now names runs and the solve is the same."""
+    item = _lattice_item((4, 6, 10, 8), 4, 6, P.F16)
+    param = P.cg_param(kappa=KAPPA, tol=1e-10, sloppy_prec=P.F16)
+    path = tmp_path / "tuned.json"
+    P.invert_cg_batch([item], param, True)
+    assert P.lib().plqcd_tune_save(str(path).encode()) == 0
+    text, out = path.read_text(), []
+    for variant in (2200, 2102):
+        lines = []
+        for line in text.splitlines():
+            for mode, v in (("plain", variant), ("xpay", 2200)):
+                if f"dslash_mrhs|p{P.F16}|r12|{mode}|n4|4x6x10x8" in line:
+                    entry = json.loads(line)
+                    entry.update(variant=v, block=64)
+                    line = json.dumps(entry)
+            lines.append(line)
+        path.write_text("\n".join(lines) + "\n")
+        assert P.lib().plqcd_tune_load(str(path).encode()) == 0
+        info, res = P.invert_cg_batch([item], param, True)
+        assert info.converged == 1
+        out.append((info.iterations, res, item["x_even"].clone(), item["x_odd"].clone()))
+    assert out[0][0] == out[1][0] and list(out[0][1]) == list(out[1][1])
+    assert all(bool((a == b).all()) for a, b in zip(out[0][2:], out[1][2:]))
+    path.write_text(text)
+    assert P.lib().plqcd_tune_load(str(path).encode()) == 0
