@@ -269,9 +269,9 @@ int launch_dslash(const Geom &g, cudaStream_t s, const DslashCall &c) {
     TuneResult known;
     if (tune_recall(id, &known)) return dispatch(g, s, c, a, known.variant, known.block);
     char key[256];
-    snprintf(key, sizeof key, "%sdslash|p%d|r%d|%s%s%s%s|%dx%dx%dx%d|n%d|c2", device_tag().c_str(), c.prec, c.recon,
+    snprintf(key, sizeof key, "%sdslash|p%d|r%d|%s%s%s%s|%dx%dx%dx%d|n%d%s", device_tag().c_str(), c.prec, c.recon,
              c.full ? "full" : "half", c.x ? "+xpay" : "", compat ? "+compat" : "", part ? "+range" : "", g.L[0],
-             g.L[1], g.L[2], g.L[3], c.nrhs);
+             g.L[1], g.L[2], g.L[3], c.nrhs, kTuneListTag);
     const int rc = tune_dslash(g, s, c, a, key);
     tune_remember(id, key);
     return rc;

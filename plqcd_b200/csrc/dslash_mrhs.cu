@@ -537,8 +537,8 @@ static int launch_mrhs_tma(const Geom &g, cudaStream_t s, const void *gauge, int
 
 // tuner key of a multi-RHS hop
 static void mrhs_key(char *key, size_t n, const Geom &g, int prec, int recon, int nrhs, bool xpay) {
-    snprintf(key, n, "%sdslash_mrhs|p%d|r%d|%s|n%d|%dx%dx%dx%d|c2", device_tag().c_str(), prec, recon,
-             xpay ? "xpay" : "plain", nrhs, g.L[0], g.L[1], g.L[2], g.L[3]);
+    snprintf(key, n, "%sdslash_mrhs|p%d|r%d|%s|n%d|%dx%dx%dx%d%s", device_tag().c_str(), prec, recon,
+             xpay ? "xpay" : "plain", nrhs, g.L[0], g.L[1], g.L[2], g.L[3], kTuneListTag);
 }
 
 // true when a launch of this multi-RHS hop would not tune (a tuned entry

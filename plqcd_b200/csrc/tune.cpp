@@ -10,8 +10,8 @@
 //   {"key": "...", "variant": V, "block": B, "ms": T}
 // Tuning is skipped (the first candidate is used) while the stream is being
 // captured into a CUDA graph, or when PLQCD_TUNE=0.
-// A key ends in the number of its candidate list ("|c2"), so an entry of an
-// older file does not hide the kernels that came since; where tuning is
+// A key ends in the number of its candidate list (kTuneListTag), so an entry
+// of an older file does not hide the kernels that came since; where tuning is
 // skipped, the entry an older file holds for the launch serves after all.
 #include <cuda_runtime.h>
 #include <sys/stat.h>
@@ -329,7 +329,7 @@ extern "C" int plqcd_tune_count(void) {
 extern "C" int plqcd_tune_get(const char *key, int *variant, int *block, double *ms) {
     plqcd::TuneResult r;
     // (a key without its candidate list's number names the launch: its entry of the present list first)
-    if (!key || (!plqcd::tune_lookup(std::string(key) + "|c2", &r) && !plqcd::tune_lookup(key, &r)))
+    if (!key || (!plqcd::tune_lookup(std::string(key) + plqcd::kTuneListTag, &r) && !plqcd::tune_lookup(key, &r)))
         return plqcd::set_error(PLQCD_ERR_ARG, "tune: no entry for key");
     if (variant) *variant = r.variant;
     if (block) *block = r.block;

@@ -23,6 +23,9 @@ int tune_launch(const std::string &key, cudaStream_t s, const std::vector<TuneRe
                 const std::function<int(const TuneResult &, bool)> &run);
 // "<device name>|" prefix for keys, so cache files do not mix GPU models
 const std::string &device_tag();
+// end of every key: the number of the families' candidate lists, raised when
+// they gain kernels
+constexpr char kTuneListTag[] = "|c2";
 bool tune_lookup(const std::string &key, TuneResult *out);
 
 // What tells the launches of the tuned families apart, as numbers: the look-up

@@ -118,3 +118,31 @@ def test_tuner_persists_choices(cuda, tmp_path):
     v, blk, ms = ctypes.c_int(), ctypes.c_int(), ctypes.c_double()
     assert P.lib().plqcd_tune_get(key.encode(), ctypes.byref(v), ctypes.byref(blk), ctypes.byref(ms)) == 0
     assert v.value in (0, 2, 3) and blk.value in (64, 128, 256) and ms.value > 0
+
+
+def test_tune_get_takes_a_launch_with_and_without_its_list_number(cuda, tmp_path):
+    """plqcd_tune_get finds a tuned hop, of one RHS and of several, by its full
+    key and by the key without the candidate list's number."""
+    import ctypes
+    L = (8, 4, 4, 6)
+    lat = new_lattice(L)
+    g = P.Gauge(lat, P.F32, 12)
+    g.random(1)
+    bs = lat.spinor_bytes(P.F32)
+    a, b = dev_bytes(2 * bs), dev_bytes(2 * bs)
+    for r in range(2):
+        lat.spinor_gaussian(a[r * bs:], P.F32, 1, 1 + r)
+    lat.dslash(g, b, a, 0, P.F32)
+    lat.dslash_mrhs(g, b, a, 2, 0, P.F32)
+    lat.synchronize()
+    path = tmp_path / "tune.json"
+    assert P.lib().plqcd_tune_save(str(path).encode()) == 0
+    keys = [line.split('"')[3] for line in path.read_text().splitlines() if "8x4x4x6" in line]
+    assert len(keys) == 2
+    v, blk, ms = ctypes.c_int(), ctypes.c_int(), ctypes.c_double()
+    for key in keys:
+        got = set()
+        for k in (key, key[:key.rindex("|c")]):
+            assert P.lib().plqcd_tune_get(k.encode(), ctypes.byref(v), ctypes.byref(blk), ctypes.byref(ms)) == 0
+            got.add((v.value, blk.value, ms.value))
+        assert len(got) == 1
