@@ -262,7 +262,7 @@ int launch_dslash(const Geom &g, cudaStream_t s, const DslashCall &c) {
         return dispatch(g, s, c, a, env_var >= 0 ? env_var : 2, block);
     }
     // a partial site range (the drop-in path's t-slab chunks) is a separate
-    // entry: the TMA kernel takes whole fields only
+    // entry: its best kernel need not be that of whole fields
     const bool part = a.h_begin != 0 || a.h_end != g.Vh;
     const TuneId id = tune_id(kTuneDslash, c.prec, c.recon, c.full | (c.x ? 2 : 0) | (compat ? 4 : 0) | (part ? 8 : 0),
                               c.nrhs, g.L);
@@ -345,15 +345,13 @@ static int tune_dslash(const Geom &g, cudaStream_t s, const DslashCall &c, const
         for (int v : {2, 3})
             for (int b : {64, 128, 256}) add(v, b);
     }
-    // TMA-staged rows: ring depth x rows per tile, where the tile fits
-    const long slab = (long)g.L0h * g.L[1] * g.L[2];  // TMA tiles cover whole t-slices
-    // (FP64 full lattice only: with loads ahead in registers the others lose
-    // at every measured size, e.g. F64 xpay at 32^3x64 295 us against 270,
-    // F32-18 full lattice 296 against 180; a near-tie is left at 16^3x32, 32.5
-    // against 32.8)
-    const bool tma_ok = c.full && c.prec == PLQCD_F64 && a.h_begin % slab == 0 && (a.h_end - a.h_begin) % slab == 0 &&
-                        getenv("PLQCD_NO_TMA") == nullptr;
-    if (tma_ok)
+    // TMA-staged rows: ring depth x rows per tile, where the tile fits, for
+    // the FP64 full lattice. (With loads ahead in registers the other forms
+    // lose at every measured size, e.g. F64 xpay at 32^3x64 295 us against
+    // 270, F32-18 full lattice 296 against 180; a near-tie is left at 16^3x32,
+    // 32.5 against 32.8. They run when the environment or an older tuning
+    // file names them.)
+    if (c.full && c.prec == PLQCD_F64 && getenv("PLQCD_NO_TMA") == nullptr)
         // (kinds 3 and 5, two own-line buffers, lost to 2 and 4 at every
         // measured point and are not tried). The own-line kernels (4, 2)
         // come first, so they keep a near-tie: they stage fewer bytes per

@@ -284,6 +284,12 @@ template <int P, int RC>
 static int launch_sum_pr(cudaStream_t s, const DslashArgs &a, const SumArgs &q, unsigned nblk, const HopSum &h) {
     using S = SpinorIO<P>;
     using L = LinkIO<P, RC>;
+    // Depth by format alone: in FP32 the two are within 2% in a solve from
+    // 12^3x24 to 32^3x64 (depth 1 0.998 to 1.002 of depth 2 with 18-real
+    // links, 8^3x16 1.03). In 16 bits depth 1 is the better one from 24^3x48
+    // on (F16 solve at 32^3x64 12.87 ms against 13.06, BF16 52.7 against
+    // 53.7), depth 2 below (F16 16^3x32 1.32 ms against 1.39, 8^3x16 0.76
+    // against 0.77); the plain hops between these choose by the tuner.
     constexpr int D = P == PLQCD_F32 ? 2 : 1, B = P == PLQCD_F64 ? 4 : P == PLQCD_F32 ? 8 : 10;
     void (*k)(const DslashArgs, const SumArgs) = nullptr;
     if (h.kind == HOP_NORM) k = k_dslash_ahead<S, L, 1, D, B, HOP_NORM>;
