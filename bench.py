@@ -48,7 +48,8 @@ BYTES_HALF_12 = 52 + 8 * 24 + 52
 # DRAM bytes (read + write) per site of one full-lattice F64 launch at 32^3x64,
 # from single-pass ncu captures of each configuration
 # (profiles/dslash_full_f64_dram_32x32x32x64.txt): variant -> bytes/site.
-# Variant 2 is the cp.async kernel, 1000*kind + 100*stages + rows a TMA kernel
+# Variant 2 is the cp.async kernel, 0 and 21 the load-ahead kernel (parities
+# apart, joined), 1000*kind + 100*stages + rows a TMA kernel
 # (kind 1: a stage per direction; 2-5: own-line rows staged once per tile).
 # 2216 is captured with the full-lattice default tile order (blocks of half
 # the z extent x all t-slices), the others with the earlier 8 x 8 (z, t)
@@ -57,6 +58,7 @@ DRAM_BYTES_PER_SITE_F64_FULL = {
     2: 2127234136 / 2097152, 1204: 2191090112 / 2097152, 2204: 2253279192 / 2097152,
     4304: 2204120856 / 2097152, 1304: 2527646688 / 2097152, 1408: 2198568976 / 2097152,
     2216: (1778083584 + 387864064) / 2097152,
+    21: (1876109312 + 390167808) / 2097152, 0: (1732283904 + 389366528) / 2097152,
 }
 
 

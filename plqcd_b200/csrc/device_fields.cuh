@@ -100,7 +100,7 @@ struct Half2<PLQCD_BF16> {
     // a bfloat16 is the upper half of its float: one operation of the ALU pipe
     // each, where a conversion takes the heavy FMA pipe, the nearest bound of
     // the 16-bit hops (8 RHS at 24^3x48 167 -> 150 us, xpay 182 -> 168; one RHS
-    // at 32^3x64 88 -> 84, full lattice 140 -> 131)
+    // at 32^3x64 88 -> 84)
     __device__ static __forceinline__ float2 unpack(uint32_t w) {
         return make_float2(__uint_as_float(__byte_perm(w, 0, 0x1044)), __uint_as_float(w & 0xffff0000u));
     }

@@ -18,15 +18,17 @@
 //   nearest bound (65% of the heavy one at 24^3x48, a third of it for the
 //   conversions), or depth 2 at 128 for small lattices.
 //
-// What bounds it, and what it measured (us, before = the best kernel so far,
-// three sets of fields in turn):
-//   F32-18 xpay 32^3x64   175 -> 135   DRAM: 6.7 TB/s of its 864 bytes per site
-//   F32-18 full 32^3x64   231 -> 180   DRAM and L2
-//   F32-12 48^3x96        571 -> 527   DRAM: 5.8 TB/s
-//   F16 xpay 32^3x64       96 -> 90    FMA pipes and latency
-//   F64-18 xpay 24^3x48    97 -> 93    DRAM: 6.2 TB/s
-//   F64-18 full 32^3x64   446 -> 441   latency at 8 warps; in a long run, where
-//                         484 -> 430   the power cap lowers the clock
+// What bounds it, and what it measured: us per launch on three sets of fields
+// in turn, in short bursts at full clock / back to back for a second, where
+// the power cap lowers the clock; before = the tuner's choice among cp.async,
+// TMA and direct loads:
+//   F32-18 xpay 32^3x64   146 / 160 -> 133 / 145   DRAM: 6.8 TB/s of its 864 bytes per site
+//   F32-18 full 32^3x64   213 / 243 -> 182 / 215   DRAM and L2
+//   F32-12 48^3x96        496 / 574 -> 483 / 561   DRAM: 6.3 / 5.5 TB/s
+//   F16 xpay 32^3x64     85.7 / 96.6 -> 86.9 / 94.4   FMA pipes and latency
+//   BF16 xpay 32^3x64    88.9 / 97.8 -> 84.1 / 90.6   the same
+//   F64-18 xpay 24^3x48  92.0 / 102.6 -> 87.2 / 94.6   DRAM: 6.6 / 6.1 TB/s
+//   F64-18 full 32^3x64   395 / 460 -> 390 / 456   latency at 8 warps
 #include <cuda_runtime.h>
 
 #include "blas.cuh"
@@ -150,9 +152,10 @@ __global__ void __launch_bounds__(1024) k_hop_sum_finish(RedScratch red, CgRepor
 // tile order: the link a parity loads for its forward term is in L1 when
 // the other one needs it for its backward term, and a tile's neighbour rows
 // are loaded by blocks that run together (F64 at 32^3x64, long run: 429 us
-// against 451 with the parities joined in the plain order and 462 in mode 2;
-// 4x2x2 430, 2x4x4 447, 4x4x4 453, 2x8x8 452, half of z x all of t 445;
-// short run 441 against 452 in mode 2).
+// against 451 with the parities joined in the plain order; 4x2x2 430, 2x4x4
+// 447, 4x4x4 453, 2x8x8 452, half of z x all of t 445). Modes 2 and 3 are a
+// near-tie that the tuner decides: 3 took 429 against 462 us on one box, 463
+// against 457 (short bursts 399 against 390) on another.
 // SUM (mode 1, whole fields): a HopSumKind; OP: the format of its output.
 // Threads past the last site compute on it and add nothing.
 template <class SIO, class LIO, int MODE, int DEPTH, int MINB, int SUM = 0, int OP = PLQCD_F64>

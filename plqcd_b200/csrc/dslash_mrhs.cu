@@ -323,10 +323,12 @@ __global__ void __launch_bounds__(256, 2) k_dslash_mrhs_pair(const MrhsArgs a) {
 
 // RHS-pair kernel with the next direction's link and two neighbour spinors
 // (at the end the two xpay operands) already on their way into registers, in
-// their stored form. 168 registers, 12 warps per SM; the heavy FMA pipe, which
-// also converts the 16-bit values, is the nearest bound. 24^3x48, 8 RHS: F16 156
-// us, where the form above takes 166 and a cp.async ring (taken out) took 170;
-// F32-18 206 both; BF16 xpay 188 against 182: the tuner decides. Links
+// their stored form. 153 to 168 registers, 12 warps per SM; the heavy FMA pipe,
+// which also converts the 16-bit values, is the nearest bound. us at 24^3x48
+// with 8 RHS, short bursts / back to back under the power cap, here against the
+// form above: F16 157 / 160, 164 / 165 (a cp.async ring, taken out, 170); F16
+// xpay 176 / 184, 179 / 184; BF16 149 / 153, 158 / 158; F32-12 xpay 201 / 229,
+// 203 / 231; but F32-18 200 / 222, 190 / 217: the tuner decides. Links
 // converted once per block and kept in shared memory as operand pairs took
 // 170: the blocks' start-up is exposed.
 constexpr int kPairAheadBlock = 64;

@@ -7,17 +7,18 @@
 // after one barrier every warp computes its RHS, the next direction's
 // neighbour spinor (and at the end the xpay operand) on its way into
 // registers meanwhile. A link crosses L2->SM once per n RHS, which with the
-// spinors is what bounds the hop: at 16^3x32 with 12 RHS and n = 2, 2.1 kB per
-// site and RHS, 12 TB/s. Same arithmetic, so the same bits, as the other
-// kernels. Threads past the last site or RHS copy in-bounds data and store
-// nothing.
+// spinors is what bounds the hop beside latency at 8 warps per SM: at 16^3x32
+// with 12 RHS and n = 2, 1.9 kB per site and RHS, 10.9 TB/s. Same arithmetic, so
+// the same bits, as the other kernels. Threads past the last site or RHS copy
+// in-bounds data and store nothing.
 //
-// Two RHS per block are best (232 registers, 8 warps per SM in 4 blocks whose
-// start-ups overlap): us at 16^3x32 with 12 RHS / 24^3x48 with 4 RHS, xpay,
-// 1: 172 / 319, 2: 134 / 240, 4: 136 / 245, 8: 173 / 385, at 200 registers 139
-// and 141 for n = 2 and 4. Before: the TMA kernel with RHS tiles 144, one
-// thread per RHS 264; links in shared memory with the spinors beside them 263 /
-// 650.
+// Two or four RHS per block (222 registers, 8 warps per SM in blocks whose
+// start-ups overlap), the tuner decides. us at 16^3x32 with 12 RHS and at
+// 24^3x48 with 4 RHS, xpay, short bursts / back to back under the power cap:
+// 2: 130 / 148 and 233 / 273, 4: 130 / 145 and 231 / 265, 8: 159 / 166; one RHS
+// per block 172 and 319 (one measurement). Before: the TMA kernel with RHS
+// tiles 142 / 157, one thread per RHS 261 / 297 at 24^3x48; links in shared
+// memory with the spinors beside them 263 and 650.
 #include <cuda_runtime.h>
 
 #include "blas.cuh"
@@ -238,6 +239,8 @@ int launch_mrhs_links_sum(const Geom &g, cudaStream_t s, const plqcd_gauge *gf, 
     q.c = static_cast<const char *>(h.c);
     q.out_fbytes = spinor_parity_bytes(g.Vh, h.out_prec);
     q.partials = partials;
+    // (two per block: four come out even where they fill it, and leave more
+    // idle warps where they don't)
     const int warps = 2, sets = h.kind == HOP_CHECK ? 2 : 1;
     PLQCD_TRY(gf->recon == 18 ? dev::launch_links<18>(g, s, m, warps, true, &q)
                               : dev::launch_links<12>(g, s, m, warps, true, &q));
