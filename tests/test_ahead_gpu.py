@@ -136,6 +136,42 @@ def test_dependent_launches_back_to_back(cuda, monkeypatch, dims, prec, recon):
     assert bool((got[0] == got[1]).all()) and bool((got[0] == got[2]).all())
 
 
+@pytest.mark.parametrize("prec,recon", [(P.F64, 18), (P.F16, 12)])
+@pytest.mark.parametrize("dims", [(4, 6, 8, 10), (16, 16, 16, 32)])
+def test_overlapped_launch_waits_for_another_stream(cuda, monkeypatch, dims, prec, recon):
+    """A launch that may overlap the one before it in its stream still waits
+    for an event of another stream queued between the two: its input is
+    written there, late, and overwritten once it has been read."""
+    import torch
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    lat = P.Lattice(dims, 0, a.cuda_stream)
+    g = P.Gauge(lat, prec, recon)
+    g.random(3)
+    nb = lat.spinor_bytes(prec)
+    n = 12
+    src, want, got = ([dev_bytes(nb) for _ in range(n)] for _ in range(3))
+    inp, busy, other = (dev_bytes(nb) for _ in range(3))
+    lat.spinor_gaussian(other, prec, 0, 7)
+    _force(monkeypatch, 0, 64)
+    for k in range(n):
+        lat.spinor_gaussian(src[k], prec, 1, 100 + k)
+        lat.dslash(g, want[k], src[k], 0, prec)
+        got[k].fill_(7)
+    torch.cuda.synchronize()
+    for k in range(n):
+        lat.dslash(g, busy, other, 1, prec)
+        with torch.cuda.stream(b):
+            torch.cuda._sleep(200000)  # (about 0.1 ms)
+            inp.copy_(src[k])
+            written = b.record_event()
+        a.wait_event(written)
+        lat.dslash(g, got[k], inp, 0, prec)
+        b.wait_event(a.record_event())
+    torch.cuda.synchronize()
+    for k in range(n):
+        assert bool((got[k] == want[k]).all()), k
+
+
 @pytest.mark.parametrize("nrhs", [2, 3])
 @pytest.mark.parametrize("prec,recon,variant", [(P.F64, 18, 4202), (P.F64, 12, 4204), (P.F32, 18, 2200),
                                                 (P.F16, 12, 2200), (P.BF16, 12, 2200)])

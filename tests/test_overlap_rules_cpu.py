@@ -37,3 +37,11 @@ def test_overlapped_kernels_are_the_known_ones():
 def test_nothing_precedes_the_wait(name):
     before = _kernels()[name].split("pdl_start()")[0]
     assert not re.findall(FORBIDDEN, before)
+
+
+@pytest.mark.parametrize("name", OVERLAPPED)
+def test_reads_are_ordinary_loads(name):
+    """Fields that a predecessor may have written don't come through the
+    non-coherent path, whose loads may move ahead of the wait (the formats'
+    own load functions take it)."""
+    assert not re.findall(r"__ldg|ld\.global\.nc|\w*IO(?:<[^>]*>)?::load(?:_raw)?\s*\(", _kernels()[name])
